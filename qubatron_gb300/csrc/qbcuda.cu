@@ -853,10 +853,47 @@ int read_stats(qbc_ctx* c, qbc_render_stats* stats, bool two) {
   return QBC_OK;
 }
 
-template <bool EXACT, bool DYN, int MODE, bool PROP>
+// Whether a launch walks with FastWalker: exact cubes, and every tree that
+// holds nodes has usable leaf boxes that all its views reach.
+bool fast_walk(const qbc_ctx* c, bool exact, int min_level) {
+  if (!exact) return false;
+  const qbc::DevScene sc = device_scene(c);
+  for (int t = 0; t < 2; ++t)
+    if ((t == 0 || sc.tree[t].n > 0) && (sc.tree[t].cbox == nullptr || min_level < sc.tree[t].box_depth)) return false;
+  return true;
+}
+
+bool fast_walk(const qbc_ctx* c, const qbc::Batch& b, bool exact) {
+  int min_level = QBC_MAX_LEVEL;
+  for (int i = 0; i < b.n; ++i) min_level = std::min(min_level, b.job[i].v.maxlevel);
+  return fast_walk(c, exact, min_level);
+}
+
+// Whether a view of the launch asks for visit counts.
+bool instrumented(const qbc::Batch& b) {
+  for (int i = 0; i < b.n; ++i)
+    if (b.job[i].o.visits) return true;
+  return false;
+}
+
+// Bit of a render kernel in qbc_ctx::attr_done.
+constexpr int kernel_variant(bool exact, bool dyn, int mode, bool prop, int walk) {
+  return (exact ? 1 : 0) + (dyn ? 2 : 0) + 4 * (mode + (prop ? 5 : 0)) + 24 * walk;
+}
+
+template <bool EXACT, bool DYN, int MODE, bool PROP, int WALK = qbc::kWalkExact>
 int launch_render(qbc_ctx* c, const qbc::Batch& b, size_t smem, const qbc::Wave& wave) {
-  auto kern = qbc::render_kernel<EXACT, DYN, MODE, PROP>;
-  const int variant = (EXACT ? 1 : 0) + (DYN ? 2 : 0) + 4 * MODE + (PROP ? 16 : 0);
+  if constexpr (EXACT && !PROP && WALK == qbc::kWalkExact) {
+    // (the shade pass counts its walks' visits)
+    if (fast_walk(c, b, EXACT)) {
+      if (MODE == qbc::kShadePass || instrumented(b))
+        return launch_render<EXACT, DYN, MODE, PROP, qbc::kWalkFastInstr>(c, b, smem, wave);
+      if constexpr (MODE != qbc::kShadePass)
+        return launch_render<EXACT, DYN, MODE, PROP, qbc::kWalkFast>(c, b, smem, wave);
+    }
+  }
+  auto kern = qbc::render_kernel<EXACT, DYN, MODE, PROP, WALK>;
+  const int variant = kernel_variant(EXACT, DYN, MODE, PROP, WALK);
   if (!(c->attr_done & (1ull << variant))) {
     QBC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
     c->attr_done |= 1ull << variant;
@@ -875,8 +912,7 @@ int launch_render(qbc_ctx* c, const qbc::Batch& b, size_t smem, const qbc::Wave&
   blocks = std::max<int64_t>(blocks, 1);
   if (tiles_only) QBC_CUDA(cudaMemsetAsync(c->queue, 0, sizeof(unsigned int), c->stream));
   qbc::DevScene sc = device_scene(c);
-  for (int i = 0; i < b.n; ++i)
-    if (b.job[i].o.visits) sc.box_words = c->wstats + qbc::kStatBoxWords;  // an instrumented render
+  if (instrumented(b)) sc.box_words = c->wstats + qbc::kStatBoxWords;
   kern<<<(unsigned)blocks, qbc::kThreads, smem, c->stream>>>(sc, b, c->queue, wave);
   QBC_CUDA(cudaGetLastError());
   ++c->launches;
@@ -887,15 +923,14 @@ int launch_render(qbc_ctx* c, const qbc::Batch& b, size_t smem, const qbc::Wave&
 template <bool EXACT, bool DYN>
 int launch_simple(qbc_ctx* c, const qbc::Batch& b, size_t smem) {
   auto kern = qbc::simple_kernel<EXACT, DYN>;
-  const int variant = 32 + (EXACT ? 1 : 0) + (DYN ? 2 : 0);
+  const int variant = 60 + (EXACT ? 1 : 0) + (DYN ? 2 : 0);
   if (!(c->attr_done & (1ull << variant))) {
     QBC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
     c->attr_done |= 1ull << variant;
   }
   const int64_t blocks = std::max<int64_t>(1, ((int64_t)b.tiles_total + 3) / 4);
   qbc::DevScene sc = device_scene(c);
-  for (int i = 0; i < b.n; ++i)
-    if (b.job[i].o.visits) sc.box_words = c->wstats + qbc::kStatBoxWords;
+  if (instrumented(b)) sc.box_words = c->wstats + qbc::kStatBoxWords;
   kern<<<(unsigned)blocks, qbc::kThreads, smem, c->stream>>>(sc, b);
   QBC_CUDA(cudaGetLastError());
   ++c->launches;
@@ -1171,9 +1206,14 @@ int render_views_impl(qbc_ctx* c, const qbc_view* views, const qbc_outputs* outs
 
 // Ray queries: one wave of resident blocks (lanes take rays by grid stride),
 // never more blocks than the rays need.
-template <bool EXACT, bool DYN>
+template <bool EXACT, bool DYN, int WALK = qbc::kWalkExact>
 int launch_rays(qbc_ctx* c, const qbc::RayJob& job, size_t smem) {
-  auto kern = qbc::rays_kernel<EXACT, DYN>;
+  if constexpr (EXACT && WALK == qbc::kWalkExact) {
+    if (fast_walk(c, EXACT, job.maxlevel))
+      return job.o.visits ? launch_rays<EXACT, DYN, qbc::kWalkFastInstr>(c, job, smem)
+                          : launch_rays<EXACT, DYN, qbc::kWalkFast>(c, job, smem);
+  }
+  auto kern = qbc::rays_kernel<EXACT, DYN, WALK>;
   int per_sm = 0;
   QBC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, qbc::kThreads, smem));
   if (per_sm < 1) return fail(QBC_E_STATE, "rays_kernel: no block fits on an SM with %zu B shared memory", smem);
@@ -1335,11 +1375,11 @@ namespace {
 // Shared-memory limit of a fused render_kernel variant, set once per context
 // (the same per-context cache launch_render uses). Setting it also loads the
 // kernel's code under lazy module loading.
-template <bool EXACT, bool DYN>
+template <bool EXACT, bool DYN, int WALK = qbc::kWalkExact>
 int fused_attr(qbc_ctx* c) {
-  const int variant = (EXACT ? 1 : 0) + (DYN ? 2 : 0);
+  const int variant = kernel_variant(EXACT, DYN, qbc::kFused, false, WALK);
   if (!(c->attr_done & (1ull << variant))) {
-    QBC_CUDA(cudaFuncSetAttribute(qbc::render_kernel<EXACT, DYN, qbc::kFused, false>,
+    QBC_CUDA(cudaFuncSetAttribute(qbc::render_kernel<EXACT, DYN, qbc::kFused, false, WALK>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
     c->attr_done |= 1ull << variant;
   }
@@ -1347,7 +1387,7 @@ int fused_attr(qbc_ctx* c) {
 }
 
 // Set-up of a no-allocation render on the context's device (current): the
-// four fused kernel variants are loaded and given their shared-memory limit
+// eight fused kernel variants are loaded and given their shared-memory limit
 // (on the context's first call; loading code can take device memory, so it
 // happens here and not in a later frame), and the counters' device address
 // is looked up with that device current. The lookup runs on every call, so
@@ -1357,6 +1397,10 @@ int noalloc_setup(qbc_ctx* c, unsigned int** out) {
   if (!rc) rc = fused_attr<true, false>(c);
   if (!rc) rc = fused_attr<false, true>(c);
   if (!rc) rc = fused_attr<false, false>(c);
+  if (!rc) rc = fused_attr<true, true, qbc::kWalkFast>(c);
+  if (!rc) rc = fused_attr<true, false, qbc::kWalkFast>(c);
+  if (!rc) rc = fused_attr<true, true, qbc::kWalkFastInstr>(c);
+  if (!rc) rc = fused_attr<true, false, qbc::kWalkFastInstr>(c);
   if (rc) return rc;
   void* ptr = nullptr;
   cudaError_t e = cudaGetSymbolAddress(&ptr, qbc_noalloc_queues);
@@ -1365,9 +1409,14 @@ int noalloc_setup(qbc_ctx* c, unsigned int** out) {
   return QBC_OK;
 }
 
-template <bool EXACT, bool DYN>
+template <bool EXACT, bool DYN, int WALK = qbc::kWalkExact>
 int launch_render_noalloc(qbc_ctx* c, const qbc::Batch& b, size_t smem, unsigned int* queue) {
-  auto kern = qbc::render_kernel<EXACT, DYN, qbc::kFused, false>;
+  if constexpr (EXACT && WALK == qbc::kWalkExact) {
+    if (fast_walk(c, b, EXACT))
+      return instrumented(b) ? launch_render_noalloc<EXACT, DYN, qbc::kWalkFastInstr>(c, b, smem, queue)
+                             : launch_render_noalloc<EXACT, DYN, qbc::kWalkFast>(c, b, smem, queue);
+  }
+  auto kern = qbc::render_kernel<EXACT, DYN, qbc::kFused, false, WALK>;
   int per_sm = 0;
   QBC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, qbc::kThreads, smem));
   if (per_sm < 1) return fail(QBC_E_STATE, "render_kernel: no block fits on an SM with %zu B shared memory", smem);

@@ -10,9 +10,11 @@
 // slowest ray of the warp.
 #pragma once
 
+#include <type_traits>
+
 #include "qbc_internal.h"
 #include "qbcuda.h"
-#include "walker.cuh"
+#include "walker_fast.cuh"
 
 namespace qbc {
 
@@ -281,14 +283,23 @@ static __device__ __noinline__ void hand_on(bool defer, int phase, uint32_t* px,
   write_record(wave.rec + (size_t)q * kSplitRecWords, px, (uint32_t)phase);
 }
 
-template <bool EXACT, bool DYN, int MODE, bool PROP>
+// The walk of a kernel. A launch takes a fast one when its basecubes are exact
+// and every tree with nodes has leaf boxes that all its views' maxlevels reach
+// (the host checks; walker_fast.cuh has the measurements), instrumented when
+// visits are counted. Inexact cubes, trees without usable boxes, pruning
+// switched off and the kernels with proposals keep walker.cuh's.
+enum Walk : int { kWalkExact = 0, kWalkFast = 1, kWalkFastInstr = 2 };
+template <bool EXACT, bool DYN, bool PROP, int WALK>
+using WalkerOf = std::conditional_t<WALK == kWalkExact, Walker<EXACT, DYN, PROP>, FastWalker<DYN, WALK == kWalkFastInstr>>;
+
+template <bool EXACT, bool DYN, int MODE, bool PROP, int WALK>
 struct Shader {
   const DevScene& sc;
   const Batch& batch;
   const Wave& wave;
   Stack st;
   PixRef px;
-  Walker<EXACT, DYN, PROP> w;
+  WalkerOf<EXACT, DYN, PROP, WALK> w;
   int phase;     // kind of the lane's current ray, kIdle without a pixel
   bool running;  // the ray is being walked
   bool enqueue;  // primary pass: the pixel goes to the shade pass
@@ -368,6 +379,15 @@ struct Shader {
     const qbc_view& v = view();
     rp = make_float3(v.light[0], v.light[1], v.light[2]);
     rd = make_float3(px.f(kPxIsp) - rp.x, px.f(kPxIsp + 1) - rp.y, px.f(kPxIsp + 2) - rp.z);
+  }
+
+  // Direction of the lane's current ray (phase), as it was started.
+  __device__ __forceinline__ float3 ray_dir() const {
+    if (phase == kPrimary) return make_float3(px.f(kPxCsv), px.f(kPxCsv + 1), px.f(kPxCsv + 2));
+    const qbc_view& v = view();
+    if (phase == kFlare)
+      return make_float3(v.light[0] - v.camfp[0], v.light[1] - v.camfp[1], v.light[2] - v.camfp[2]);
+    return make_float3(px.f(kPxIsp) - v.light[0], px.f(kPxIsp + 1) - v.light[1], px.f(kPxIsp + 2) - v.light[2]);
   }
 
   // The next usable proposal from prop_k on: the level-pdepth cell around
@@ -516,7 +536,8 @@ struct Shader {
     if (r == kLeaf) {
       int32_t ms, md;
       w.leaf(sc, ms, md, col, nrm);
-      isp = w.e;
+      if constexpr (WALK != kWalkExact) isp = w.leaf_point(st, bc, ray_dir());
+      else isp = w.e;
     }
 
     if (phase == kProposal) {
@@ -663,14 +684,14 @@ constexpr int render_min_blocks() {
   return (MODE == kShadePass || (DYN && !EXACT)) ? (DYN ? 5 : 1) : 6;
 }
 
-template <bool EXACT, bool DYN, int MODE, bool PROP>
+template <bool EXACT, bool DYN, int MODE, bool PROP, int WALK>
 __global__ void __launch_bounds__(kThreads, render_min_blocks<EXACT, DYN, MODE>()) render_kernel(DevScene sc, const __grid_constant__ Batch batch,
                                                           unsigned int* queue, const __grid_constant__ Wave wave) {
   extern __shared__ uint32_t smem[];
   const int tid = threadIdx.x, lane = tid & 31;
-  constexpr int kW = Walker<EXACT, DYN, PROP>::kWords;
+  constexpr int kW = WalkerOf<EXACT, DYN, PROP, WALK>::kWords;
   constexpr bool kRecords = MODE == kShadePass || MODE == kSplitFinish;
-  Shader<EXACT, DYN, MODE, PROP> S{sc, batch, wave, Stack{smem + tid, kThreads},
+  Shader<EXACT, DYN, MODE, PROP, WALK> S{sc, batch, wave, Stack{smem + tid, kThreads},
                                    PixRef{smem + kW * batch.max_level * kThreads + tid}};
   S.phase = kIdle;
   S.running = false;
@@ -772,9 +793,11 @@ __global__ void __launch_bounds__(kThreads, render_min_blocks<EXACT, DYN, MODE>(
           defer = true;
         } else {
           S.running = true;
-          if (PROP && S.phase == kProposal) {
-            S.w.target = S.next_target;
-            S.w.tdepth = S.next_tdepth;
+          if constexpr (PROP) {
+            if (S.phase == kProposal) {
+              S.w.target = S.next_target;
+              S.w.tdepth = S.next_tdepth;
+            }
           }
         }
       }
@@ -784,11 +807,13 @@ __global__ void __launch_bounds__(kThreads, render_min_blocks<EXACT, DYN, MODE>(
       }
       // whether every running lane may divide by its reciprocals (the set
       // of running rays changes only here)
-      fast = EXACT && __all_sync(0xFFFFFFFFu, !S.running || (S.w.mode & 1u));
+      if constexpr (EXACT && WALK == kWalkExact) fast = __all_sync(0xFFFFFFFFu, !S.running || (S.w.mode & 1u));
       if (exhausted && __ballot_sync(0xFFFFFFFFu, S.phase != kIdle) == 0) break;
     }
     if (S.running) {
-      const int r = S.w.step(sc, S.maxlevel, S.bc, S.st, fast);
+      int r;
+      if constexpr (WALK == kWalkExact) r = S.w.step(sc, S.maxlevel, S.bc, S.st, fast);
+      else r = S.w.step(sc, S.maxlevel, S.bc, S.st, [&] { return S.ray_dir(); });
       if (r != kRunning) {
         S.running = false;
         S.result = r;
@@ -821,7 +846,7 @@ __global__ void __launch_bounds__(kThreads, render_min_blocks<EXACT, DYN, kFused
   if (tile >= batch.tiles_total) return;
   constexpr int kW = Walker<EXACT, DYN, false>::kWords;
   const Wave wave{};
-  Shader<EXACT, DYN, kFused, false> S{sc, batch, wave, Stack{smem + tid, kThreads},
+  Shader<EXACT, DYN, kFused, false, kWalkExact> S{sc, batch, wave, Stack{smem + tid, kThreads},
                                       PixRef{smem + kW * batch.max_level * kThreads + tid}};
   S.running = false;
   S.enqueue = false;
@@ -867,16 +892,17 @@ struct RayJob {
 // until service_min lanes of its warp wait (or none runs), then they write
 // their results and start their next rays together, and the warp votes on
 // the division by reciprocals for the rays now running.
-template <bool EXACT, bool DYN>
+template <bool EXACT, bool DYN, int WALK>
 __global__ void __launch_bounds__(kThreads) rays_kernel(DevScene sc, const __grid_constant__ RayJob job) {
   extern __shared__ uint32_t smem[];
   Stack st{smem + threadIdx.x, kThreads};
-  Walker<EXACT, DYN> w;
+  WalkerOf<EXACT, DYN, false, WALK> w;
   const int64_t stride = (int64_t)gridDim.x * kThreads;
   int64_t i = blockIdx.x * (int64_t)kThreads + threadIdx.x;  // the lane's current ray
   int r = kMiss;
   bool running = false, ended = false;  // ended: ray i is done and not yet written
   bool fast = false;                    // warp-uniform
+  auto ray_dir = [&] { return make_float3(job.dir[3 * i], job.dir[3 * i + 1], job.dir[3 * i + 2]); };
   for (;;) {
     const unsigned run = __ballot_sync(0xFFFFFFFFu, running);
     if (run == 0u || 32 - __popc(run) >= job.service_min) {
@@ -887,7 +913,8 @@ __global__ void __launch_bounds__(kThreads) rays_kernel(DevScene sc, const __gri
             float4 col = make_float4(0.f, 0.f, 0.f, 0.f), nrm = col, isp = col;
             if (r == kLeaf) {
               w.leaf(sc, ms, md, col, nrm);
-              isp = w.e;
+              if constexpr (WALK != kWalkExact) isp = w.leaf_point(st, job.bc, ray_dir());
+              else isp = w.e;
               ls = w.ns;
               ld = w.nd;
             }
@@ -915,10 +942,11 @@ __global__ void __launch_bounds__(kThreads) rays_kernel(DevScene sc, const __gri
         }
       }
       if (__ballot_sync(0xFFFFFFFFu, running) == 0u) break;  // no ray left for any lane
-      fast = EXACT && __all_sync(0xFFFFFFFFu, !running || (w.mode & 1u));
+      if constexpr (EXACT && WALK == kWalkExact) fast = __all_sync(0xFFFFFFFFu, !running || (w.mode & 1u));
     }
     if (running) {
-      r = w.step(sc, job.maxlevel, job.bc, st, fast);
+      if constexpr (WALK == kWalkExact) r = w.step(sc, job.maxlevel, job.bc, st, fast);
+      else r = w.step(sc, job.maxlevel, job.bc, st, ray_dir);
       if (r != kRunning) {
         running = false;
         ended = true;
