@@ -856,7 +856,7 @@ int read_stats(qbc_ctx* c, qbc_render_stats* stats, bool two) {
 // Whether a launch walks with FastWalker: exact cubes, and every tree that
 // holds nodes has usable leaf boxes that all its views reach.
 bool fast_walk(const qbc_ctx* c, bool exact, int min_level) {
-  if (!exact) return false;
+  if (!exact || min_level < 1) return false;
   const qbc::DevScene sc = device_scene(c);
   for (int t = 0; t < 2; ++t)
     if ((t == 0 || sc.tree[t].n > 0) && (sc.tree[t].cbox == nullptr || min_level < sc.tree[t].box_depth)) return false;

@@ -13,17 +13,17 @@
 // shader's arithmetic from the exact entry point, for this cube and the
 // subtree below it (0.05-0.2 % of the visits).
 //
-// What bounds it: instruction issue (68 % of the cycles, ALU pipe 66 % busy;
-// DRAM below 2 % of its rate). The exact subnode test, filter and descent took
-// 4.4G warp instructions for a 1920x1080 view of a 5M-point room; this walk
-// takes 3.2G. A step has no divergent branch but the ambiguous one: all four
-// list entries are tested at once, with the two bounds of an axis in one
-// packed FMA, and a descent reads its own list back from the stack as a pop
-// does (with branches around both, a view took 4.2 ms; without, 3.9).
-// 16 x 1080p of a 20M-point room: 69.2 -> 44.7 ms; 1200x800 of a 5M-point
-// room 2.08 -> 1.39 ms; 320x240 of a 200K-point floor 0.23 -> 0.16 ms; 4M
-// random rays 5.73 -> 4.33 ms. 6 blocks of 128 threads per SM (79 registers);
-// 7 (18 bytes spilled) measured the same, 8 spill 94 bytes and take 1.6x.
+// What bounds it: the ALU pipe (71 % busy) and instruction issue (68 % of the
+// cycles; DRAM below 2 % of its rate). With the exact subnode test, filter
+// and descent a 1920x1080 view of a 5M-point room took 4.4G warp
+// instructions; this walk takes 3.0G. A step has no divergent branch but the
+// ambiguous one: all four list entries are read and tested at once, the two
+// bounds of an axis in one packed FMA, and a descent reads its own list back
+// from the stack as a pop does (with branches around both, a view took 4.2
+// ms; without, 3.9). 16 x 1080p of a 20M-point room: 68.8 -> 44.7 ms, 37.8
+// with the service phase of render.cuh lightened as well; 4M random rays
+// 5.7 -> 4.2 ms. 6 blocks of 128 threads per SM (79 registers); 7 (18 bytes
+// spilled) measured the same, 8 spill 94 bytes and take 1.6x.
 //
 // Path. The corner of the current cube is held per axis as the float 1 + path
 // bits (bit 22 - k for level k), so fma(X, S, -S) is the exact coordinate, a
@@ -155,34 +155,27 @@ static __device__ __noinline__ uint32_t words_read(const int32_t* child, int32_t
   return nw;
 }
 
-// Two values by one packed operation: f.x * u + c.x, f.y * u + c.y.
-__device__ __forceinline__ float2 fma2(float2 f, float u, float2 c) {
-  float2 r;
-  asm("{\n"
-      ".reg .b64 a, b, c, d;\n"
-      "mov.b64 a, {%2, %3};\n"
-      "mov.b64 b, {%4, %4};\n"
-      "mov.b64 c, {%5, %6};\n"
-      "fma.rn.f32x2 d, a, b, c;\n"
-      "mov.b64 {%0, %1}, d;\n"
-      "}"
-      : "=f"(r.x), "=f"(r.y)
-      : "f"(f.x), "f"(f.y), "f"(u), "f"(c.x), "f"(c.y));
+// Pairs of floats for the packed operations: f.x * u.x + c.x, f.y * u.y + c.y
+// (held as 64-bit registers: a pair used more than once is built once).
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pair(float x, float y) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
   return r;
 }
-
-// a.x + b.x, a.y + b.y by one packed operation.
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+__device__ __forceinline__ float2 unpair(f2 v) {
   float2 r;
-  asm("{\n"
-      ".reg .b64 a, b, d;\n"
-      "mov.b64 a, {%2, %3};\n"
-      "mov.b64 b, {%4, %5};\n"
-      "add.rn.f32x2 d, a, b;\n"
-      "mov.b64 {%0, %1}, d;\n"
-      "}"
-      : "=f"(r.x), "=f"(r.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
 
@@ -252,15 +245,29 @@ struct FastWalker {
     selz = selector(2u, inv.z > 0.0f ? 1u : 0u);
     const float mi = fmaxf(fabsf(inv.x), fmaxf(fabsf(inv.y), fabsf(inv.z)));
     guard = 7.4505806e-08f * (s * mi);  // 1.25 * 2^-24
-    float4 h0;
-    if (!base_entry(p, d, s, h0)) return kDiscard;
-    // the parametric test takes the ray's largest t at the near faces for the
-    // entry t: at a basecube edge the shader may have picked another face
-    const float nx = fminf((0.0f - p.x) * inv.x, (s - p.x) * inv.x);
-    const float ny = fminf((0.0f - p.y) * inv.y, (s - p.y) * inv.y);
-    const float nz = fminf((0.0f - p.z) * inv.z, (s - p.z) * inv.z);
-    const float t0 = fmaxf(fmaxf(nx, 0.0f), fmaxf(ny, nz));
-    slow = !geo || !(fabsf(h0.w - t0) <= __fmaf_rn(t0, kRelGuard, guard));
+    // The basecube's faces by t: where no two of the t values that decide are
+    // closer than the errors, the shader's face tests pass for the entry and
+    // the exit face alone, or (a miss, or the cube behind the origin) it
+    // discards. Else its own arithmetic decides: six face hits, each with a
+    // division (for nearly every ray they were the start's largest part).
+    const float x0 = (0.0f - p.x) * inv.x, x1 = (s - p.x) * inv.x;
+    const float y0 = (0.0f - p.y) * inv.y, y1 = (s - p.y) * inv.y;
+    const float z0 = (0.0f - p.z) * inv.z, z1 = (s - p.z) * inv.z;
+    const float nx = fminf(x0, x1), ny = fminf(y0, y1), nz = fminf(z0, z1);
+    const float fx = fmaxf(x0, x1), fy = fmaxf(y0, y1), fz = fmaxf(z0, z1);
+    const float t0 = fmaxf(fmaxf(nx, ny), nz), t1 = fminf(fminf(fx, fy), fz);
+    const float n2 = fmaxf(fminf(nx, ny), fminf(fmaxf(nx, ny), nz));  // the second near and far t
+    const float f2 = fminf(fmaxf(fx, fy), fmaxf(fminf(fx, fy), fz));
+    const float g = __fmaf_rn(fmaxf(fabsf(t0), fabsf(t1)), kRelGuard, guard);
+    if (geo && (t0 > t1 + g || t1 < -g)) return kDiscard;
+    slow = !geo;
+    if (!(geo && t1 > t0 + g && t1 > g && t0 - n2 > g && f2 - t1 > g && fabsf(t0) > g)) {
+      float4 h0;
+      if (!base_entry(p, d, s, h0)) return kDiscard;
+      // the walk takes the largest near t for the entry t: at a basecube edge
+      // the shader may have picked another face
+      slow |= !(fabsf(h0.w - fmaxf(t0, 0.0f)) <= g);
+    }
     return kRunning;
   }
 
@@ -279,10 +286,10 @@ struct FastWalker {
   // dir() gives the ray's direction. Returns kRunning, kLeaf or kMiss.
   template <class Dir>
   __device__ __forceinline__ int step(const DevScene& sc, int maxlevel, float4 bc, const Stack& st, Dir dir) {
-    if (maxlevel == 0) return kLeaf;
     const float s = bc.w;
+    // trees with a node at this cube (none at maxlevel: see the end)
     const bool dl = DYN && !(mode & 8u);
-    const bool has_s = DYN ? ns > 0 || level == 0 : ns >= 0;
+    const bool has_s = DYN ? ns > 0 || level == 0 : level < maxlevel;
     const bool has_d = dl && (nd > 0 || level == 0);
     if (INSTR) {
       if (has_s) ++vis_s;
@@ -290,6 +297,7 @@ struct FastWalker {
     }
 
     // ---- the ray's t at the cube's planes (box_frame's terms) ----
+    const bool geo = (mode & 2u) != 0u;
     const float lv2 = __int_as_float((127 - level) << 23);  // 2^-level
     const float ax = (path_up(X, s) - p.x) * inv.x;
     const float ay = (path_down(Y, s) - p.y) * inv.y;
@@ -346,14 +354,14 @@ struct FastWalker {
     }
 
     // ---- leaf boxes of the listed children ----
-    float2 cx, cy, cz;  // near and far terms of a bound
+    f2 cx, cy, cz;  // near and far terms of a bound
     if (INSTR) {
       // child_box_hit's a0 and a1, the near one first
       const float m = s * 6.1035156e-05f;  // 2^-14 S
       const float mx = fabsf(m * inv.x), my = fabsf(m * inv.y), mz = fabsf(m * inv.z);
-      cx = make_float2(ax - mx, ax + mx);
-      cy = make_float2(ay - my, ay + my);
-      cz = make_float2(az - mz, az + mz);
+      cx = pair(ax - mx, ax + mx);
+      cy = pair(ay - my, ay + my);
+      cz = pair(az - mz, az + mz);
     } else {
       // a bound's float is 2^15 + units, a high bound's cell ends one unit
       // later (half a unit either way from the middle), and 2^-14 S is
@@ -361,57 +369,57 @@ struct FastWalker {
       const float k = 0.51f + __int_as_float((127 - 5 + level) << 23);
       const float bx = __fmaf_rn(ux, -32767.5f, ax), by = __fmaf_rn(uy, -32767.5f, ay),
                   bz = __fmaf_rn(uz, -32767.5f, az);
-      cx = make_float2(__fmaf_rn(fabsf(ux), -k, bx), __fmaf_rn(fabsf(ux), k, bx));
-      cy = make_float2(__fmaf_rn(fabsf(uy), -k, by), __fmaf_rn(fabsf(uy), k, by));
-      cz = make_float2(__fmaf_rn(fabsf(uz), -k, bz), __fmaf_rn(fabsf(uz), k, bz));
+      cx = pair(__fmaf_rn(fabsf(ux), -k, bx), __fmaf_rn(fabsf(ux), k, bx));
+      cy = pair(__fmaf_rn(fabsf(uy), -k, by), __fmaf_rn(fabsf(uy), k, by));
+      cz = pair(__fmaf_rn(fabsf(uz), -k, bz), __fmaf_rn(fabsf(uz), k, bz));
     }
+    const f2 u2x = pair(ux, ux), u2y = pair(uy, uy), u2z = pair(uz, uz);
     auto meets = [&](uint2 r, uint32_t oct) {
       // bytes 0, 1, 2: the octet's x, y, z bit; byte 3: the exponent
       const uint32_t b = ((oct * 0x4081u) & 0x00010101u) | (INSTR ? 0x4B000000u : 0x47000000u);
-      float2 qx = make_float2(__uint_as_float(prmt(r.x, b, selx)), __uint_as_float(prmt(r.x, b, selx ^ kBound)));
-      float2 qy = make_float2(__uint_as_float(prmt(r.x, b, sely)), __uint_as_float(prmt(r.x, b, sely ^ kBound)));
-      float2 qz = make_float2(__uint_as_float(prmt(r.y, b, selz)), __uint_as_float(prmt(r.y, b, selz ^ kBound)));
+      auto bounds = [&](uint32_t w, uint32_t sel) {
+        return pair(__uint_as_float(prmt(w, b, sel)), __uint_as_float(prmt(w, b, sel ^ kBound)));
+      };
+      f2 qx = bounds(r.x, selx), qy = bounds(r.x, sely), qz = bounds(r.y, selz);
       if (INSTR) {
         // a high bound (an odd byte): one unit more
         auto off = [](uint32_t sel) {
           const float k = (sel & 1u) ? -8388607.0f : -8388608.0f;
-          return make_float2(k, -16777215.0f - k);
+          return pair(k, -16777215.0f - k);
         };
         qx = add2(qx, off(selx));
         qy = add2(qy, off(sely));
         qz = add2(qz, off(selz));
       }
-      qx = fma2(qx, ux, cx);
-      qy = fma2(qy, uy, cy);
-      qz = fma2(qz, uz, cz);
-      const float tn = fmaxf(fmaxf(qx.x, qy.x), qz.x), tf = fminf(fminf(qx.y, qy.y), qz.y);
+      const float2 tx = unpair(fma2(qx, u2x, cx)), ty = unpair(fma2(qy, u2y, cy)), tz = unpair(fma2(qz, u2z, cz));
+      const float tn = fmaxf(fmaxf(tx.x, ty.x), tz.x), tf = fminf(fminf(tx.y, ty.y), tz.y);
       return (tn <= tf) & (tf >= 0.0f);
     };
-    const bool geo = (mode & 2u) != 0u;
     // entries of a tree's node: the children with leaves (an empty child's
     // record says so) whose box the ray meets; the deepest level's children
-    // are leaf cells, which every listed entry meets
+    // are leaf cells, which every listed entry meets. All four records are
+    // read and tested, listed or not: they are in two sectors anyhow, and the
+    // lanes of a warp nearly always list four between them.
     auto filter = [&](const DevTree& t, int32_t node) {
-      uint32_t keep = 0u;
-      if (level >= t.box_depth) return keep;
-      if (__builtin_expect(!geo, 0)) {  // the shader's own test (octree_fsh.c:313-317)
-        const int32_t* c = reinterpret_cast<const int32_t*>(t.child) + 8 * (size_t)(uint32_t)node;
-        for (int i = 0; i < 4; ++i)
-          if (v[i] && __ldg(c + ((pk >> (5 * i)) & 7u)) > 0) keep |= 1u << i;
-        return keep;
-      }
       const uint2* rec = reinterpret_cast<const uint2*>(t.cbox) + (size_t)(uint32_t)node * 8;
       const bool any = level + 1 == t.box_depth;
       uint2 r[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) r[i] = v[i] ? __ldg(rec + o[i]) : make_uint2(kEmptyBox, 0u);
+      for (int i = 0; i < 4; ++i) r[i] = __ldg(rec + o[i]);
+      uint32_t keep = 0u;
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if ((r[i].x != kEmptyBox) & (any | meets(r[i], o[i]))) keep |= 1u << i;
-      return keep;
+      for (int i = 0; i < 4; ++i) keep |= (v[i] & (r[i].x != kEmptyBox) & (any | meets(r[i], o[i]))) ? 1u << i : 0u;
+      if (__builtin_expect(!geo, 0)) {  // the shader's own test (octree_fsh.c:313-317)
+        const int32_t* c = reinterpret_cast<const int32_t*>(t.child) + 8 * (size_t)(uint32_t)node;
+        keep = 0u;
+        for (int i = 0; i < 4; ++i)
+          if (v[i] && __ldg(c + ((pk >> (5 * i)) & 7u)) > 0) keep |= 1u << i;
+      }
+      return level < t.box_depth ? keep : 0u;
     };
     uint32_t ks = 0u, kd = 0u;
-    if (has_s) ks = filter(sc.tree[0], ns);
+    if (!DYN) ks = filter(sc.tree[0], ns);
+    else if (has_s) ks = filter(sc.tree[0], ns);
     if (DYN && has_d) kd = filter(sc.tree[1], nd);
     if (INSTR && sc.box_words) {
       const int n = 1 + (int)v[1] + (int)v[2] + (int)v[3];
@@ -429,7 +437,7 @@ struct FastWalker {
     // read back, also where that is this one: descending and popping lanes
     // follow one sequence without a branch.
     const uint32_t all = DYN ? ks | kd : ks;
-    if (all) {  // (the level of a removed leaf's step may lie past the stack)
+    if (all) {
       slot(st, level, 0) = pk | (ks << 20) | (DYN ? kd << 24 : 0u) | (exact ? 1u << 30 : 0u);
       slot(st, level, 1) = (uint32_t)ns;
       if (DYN) slot(st, level, 2) = (uint32_t)nd;
@@ -463,12 +471,13 @@ struct FastWalker {
     Y = (Y & keep) | ((oct & 2) ? bit : 0u);
     Z = (Z & keep) | ((oct & 4) ? bit : 0u);
     slow = (pk >> 30) != 0u;
-    level = lv + 1;
-    // a removed leaf's link is cut while its box stays: such a child lists
-    // nothing in the next step
-    ns = ok ? cs : -1;
-    nd = !DYN ? 0 : (ok ? cd : -1);
-    return ok && level == maxlevel ? kLeaf : kRunning;
+    // a removed node's link is cut while its box stays: the lane goes on from
+    // the root's record at maxlevel, at and below every tree's depth, where
+    // the filter lists nothing, so its next step takes another entry
+    level = ok ? lv + 1 : maxlevel;
+    ns = ok ? cs : 0;
+    nd = ok ? cd : 0;
+    return ok & (level == maxlevel) ? kLeaf : kRunning;
   }
 
   // Entry point of the leaf cell; call after step() returned kLeaf.

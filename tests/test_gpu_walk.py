@@ -101,3 +101,22 @@ def test_cameras_on_bisecting_planes(oracle, scene, character, two_trees):
             counted = ctx.render_host([v], streams + ("visits",))[0].arrays
             compare_frame(counted, ref, f"{pos}", visits=True)
             compare_frame({**plain, "visits": counted["visits"]}, ref, f"{pos} without visits")
+            # bytes alone are shaded by another route
+            assert np.array_equal(ctx.render_host([v], ("rgba8",))[0]["rgba8"], ref["rgba8"]), pos
+
+
+@pytest.mark.parametrize("shoot", [0, 1, 2, -1])
+def test_bytes_alone(oracle, scene, shoot):
+    """A frame of bytes alone where its shading must fall back: texels beyond
+    [0, 1], zero, tiny, huge and non-finite normals, shoot outside 0 and 1."""
+    import qubatron_gb300 as qb
+    rng = np.random.default_rng(3)
+    n = scene.colors.shape[0]
+    col = scene.colors * rng.choice([0.0, 1.0, -1.0, 3.0, 1e4], (n, 3), p=[0.1, 0.6, 0.1, 0.1, 0.1]).astype(np.float32)
+    nrm = scene.normals * rng.choice([1.0, 0.0, 1e-20, 1e20, 1e-30, np.inf, np.nan], (n, 1),
+                                     p=[0.4, 0.1, 0.1, 0.1, 0.1, 0.1, 0.1]).astype(np.float32)
+    v = qb.view_setup(201, 113, (903.7, 421.3, 1302.9), (0.2, -0.3, 0.0), 0.4, 10, LEVELS, S, shoot, 0.0)
+    ref = oracle.render(oracle_scene(oracle, scene.nodes, col, nrm), oracle.QboView.from_bytes(v.to_bytes()))
+    with qb.OctreeGLC(0) as ctx:
+        upload_scene(ctx, scene.nodes, col, nrm)
+        assert np.array_equal(ctx.render_host([v], ("rgba8",))[0]["rgba8"], ref["rgba8"])
