@@ -883,7 +883,7 @@ constexpr int kernel_variant(bool exact, bool dyn, int mode, bool prop, int walk
 
 template <bool EXACT, bool DYN, int MODE, bool PROP, int WALK = qbc::kWalkExact>
 int launch_render(qbc_ctx* c, const qbc::Batch& b, size_t smem, const qbc::Wave& wave) {
-  if constexpr (EXACT && !PROP && WALK == qbc::kWalkExact) {
+  if constexpr (EXACT && WALK == qbc::kWalkExact) {
     // (the shade pass counts its walks' visits)
     if (fast_walk(c, b, EXACT)) {
       if (MODE == qbc::kShadePass || instrumented(b))

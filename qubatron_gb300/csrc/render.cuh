@@ -302,11 +302,12 @@ static __device__ __noinline__ void hand_on(bool defer, int phase, uint32_t* px,
 // The walk of a kernel. A launch takes a fast one when its basecubes are exact
 // and every tree with nodes has leaf boxes that all its views' maxlevels reach
 // (the host checks; walker_fast.cuh has the measurements), instrumented when
-// visits are counted. Inexact cubes, trees without usable boxes, pruning
-// switched off and the kernels with proposals keep walker.cuh's.
+// visits are counted (so in every shade pass, whose statistics count them).
+// Inexact cubes, trees without usable boxes and pruning switched off keep
+// walker.cuh's.
 enum Walk : int { kWalkExact = 0, kWalkFast = 1, kWalkFastInstr = 2 };
 template <bool EXACT, bool DYN, bool PROP, int WALK>
-using WalkerOf = std::conditional_t<WALK == kWalkExact, Walker<EXACT, DYN, PROP>, FastWalker<DYN, WALK == kWalkFastInstr>>;
+using WalkerOf = std::conditional_t<WALK == kWalkExact, Walker<EXACT, DYN, PROP>, FastWalker<DYN, WALK == kWalkFastInstr, PROP>>;
 
 template <bool EXACT, bool DYN, int MODE, bool PROP, int WALK>
 struct Shader {
@@ -326,7 +327,7 @@ struct Shader {
   uint32_t next_target;
   int next_tdepth;
   float4 bc;
-  unsigned long long stat[kStatCount];
+  uint32_t stat[kStatCount];  // of this lane (2^32 visits of one lane would take an hour)
 
   __device__ __forceinline__ const qbc_view& view() const { return batch.job[px.w(kPxView)].v; }
 
@@ -742,14 +743,17 @@ constexpr int kServiceMinDefault = 4;
 // nothing (or next to nothing) spills: 6 (80 registers) for the fused,
 // primary-pass and split kernels; the shade passes, which also shade and
 // test proposals, and the two-tree walk of an inexact basecube (which keeps
-// the node blocks live) keep 5 with both trees and no bound with one.
-template <bool EXACT, bool DYN, int MODE>
+// the node blocks live) keep 5 with both trees and, on the exact walk, no
+// bound with one (the fast walk's shade pass with proposals at 6 blocks
+// spills 72 bytes and takes 5.20 instead of 5.17 ms a frame of 4 x 1080p).
+template <bool EXACT, bool DYN, int MODE, int WALK>
 constexpr int render_min_blocks() {
+  if (WALK != kWalkExact) return MODE == kShadePass ? 5 : 6;
   return (MODE == kShadePass || (DYN && !EXACT)) ? (DYN ? 5 : 1) : 6;
 }
 
 template <bool EXACT, bool DYN, int MODE, bool PROP, int WALK>
-__global__ void __launch_bounds__(kThreads, render_min_blocks<EXACT, DYN, MODE>()) render_kernel(DevScene sc, const __grid_constant__ Batch batch,
+__global__ void __launch_bounds__(kThreads, render_min_blocks<EXACT, DYN, MODE, WALK>()) render_kernel(DevScene sc, const __grid_constant__ Batch batch,
                                                           unsigned int* queue, const __grid_constant__ Wave wave) {
   extern __shared__ uint32_t smem[];
   __shared__ int3 corner[kThreads / 32];  // per warp: view and first pixel of its tile
@@ -911,7 +915,7 @@ __global__ void __launch_bounds__(kThreads, render_min_blocks<EXACT, DYN, MODE>(
 // render_kernel, so the same pixels; kept as the baseline the persistent
 // kernel is measured against.
 template <bool EXACT, bool DYN>
-__global__ void __launch_bounds__(kThreads, render_min_blocks<EXACT, DYN, kFused>()) simple_kernel(DevScene sc, const __grid_constant__ Batch batch) {
+__global__ void __launch_bounds__(kThreads, render_min_blocks<EXACT, DYN, kFused, kWalkExact>()) simple_kernel(DevScene sc, const __grid_constant__ Batch batch) {
   extern __shared__ uint32_t smem[];
   const int tid = threadIdx.x;
   const int tile = (int)((blockIdx.x * (unsigned)kThreads + tid) >> 5);

@@ -184,7 +184,7 @@ __device__ __forceinline__ f2 add2(f2 a, f2 b) {
 // walk in walker.cuh. The others use a cheaper box test within the same
 // margin, and descend into a tree only where its own box is met. The leaves
 // are the same.
-template <bool DYN, bool INSTR>
+template <bool DYN, bool INSTR, bool PROP = false>
 struct FastWalker {
   float3 p;      // ray origin
   float3 inv;    // RN(1 / d) per component of the direction (0 for a zero component)
@@ -201,6 +201,11 @@ struct FastWalker {
   bool slow;                  // this cube lies below an ambiguous one (or the ray allows no boxes)
   bool oob;
   uint32_t vis_s, vis_d;
+  // proposal test (PROP only): above tdepth the walk takes only the first
+  // entry towards the cell of path `target` (3 bits per level, root first);
+  // no entries are left there, so pops stop at tdepth
+  uint32_t target;
+  int tdepth;
 
   static constexpr int kWords = DYN ? 3 : 2;
   static constexpr uint32_t kEmptyBox = 0x00FF00FFu;  // word x of a child without leaves
@@ -230,6 +235,8 @@ struct FastWalker {
     oob = false;
     vis_s = 0;
     vis_d = 0;
+    target = 0u;
+    tdepth = 0;
     const float s = bc.w;
     const bool fdiv = recip_div_ok(p, d, s);
     const bool geo = box_ray_ok(p, d, s, fdiv);
@@ -436,6 +443,16 @@ struct FastWalker {
     // The list goes to the stack and the nearest level with entries left is
     // read back, also where that is this one: descending and popping lanes
     // follow one sequence without a branch.
+    if (PROP && level < tdepth) {
+      const uint32_t want = target >> (3 * (tdepth - 1 - level));
+      uint32_t to = 0u;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) to |= (((pk >> (5 * i)) ^ want) & 7u) == 0u ? 1u << i : 0u;
+      to &= ks | kd;
+      to &= 0u - to;  // the first
+      ks &= to;
+      kd &= to;
+    }
     const uint32_t all = DYN ? ks | kd : ks;
     if (all) {
       slot(st, level, 0) = pk | (ks << 20) | (DYN ? kd << 24 : 0u) | (exact ? 1u << 30 : 0u);

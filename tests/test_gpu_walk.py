@@ -113,8 +113,9 @@ def test_bytes_alone(oracle, scene, shoot):
     rng = np.random.default_rng(3)
     n = scene.colors.shape[0]
     col = scene.colors * rng.choice([0.0, 1.0, -1.0, 3.0, 1e4], (n, 3), p=[0.1, 0.6, 0.1, 0.1, 0.1]).astype(np.float32)
-    nrm = scene.normals * rng.choice([1.0, 0.0, 1e-20, 1e20, 1e-30, np.inf, np.nan], (n, 1),
-                                     p=[0.4, 0.1, 0.1, 0.1, 0.1, 0.1, 0.1]).astype(np.float32)
+    with np.errstate(invalid="ignore"):
+        nrm = scene.normals * rng.choice([1.0, 0.0, 1e-20, 1e20, 1e-30, np.inf, np.nan], (n, 1),
+                                         p=[0.4, 0.1, 0.1, 0.1, 0.1, 0.1, 0.1]).astype(np.float32)
     v = qb.view_setup(201, 113, (903.7, 421.3, 1302.9), (0.2, -0.3, 0.0), 0.4, 10, LEVELS, S, shoot, 0.0)
     ref = oracle.render(oracle_scene(oracle, scene.nodes, col, nrm), oracle.QboView.from_bytes(v.to_bytes()))
     with qb.OctreeGLC(0) as ctx:
