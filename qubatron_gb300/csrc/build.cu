@@ -12,29 +12,48 @@
 // Node ids follow from one prefix sum over points in index order:
 //   id(i, l) = 1 + sum_{j < i} (levels - c_j + 1) + (l - c_i).
 //
-// Creators, level by level, with one kernel per level: the level-l group of
-// a point is (creator of its level-(l-1) node, its level-l octet), a slot
-// creator * 8 + octet of a table the points atomicMin their index into; the
-// next kernel reads the winner. Warps merge equal slots first (their lanes'
-// indices increase, so the lowest lane of a group holds its minimum). The
-// top levels, whose few groups every block meets, use tables indexed by the
-// prefix itself, reduced in shared memory per block first. The deeper
-// levels rotate three tables of 8 entries per point; a table's entries are
-// reset to "empty" by the kernel two levels later, so the tables are empty
-// again when the build ends.
+// Creators, level by level: the level-l group of a point is (creator of its
+// level-(l-1) node, its level-l octet), a slot creator * 8 + octet of a table
+// the points atomicMin their index into; the next kernel reads the winner. A
+// run of lanes with one slot proposes once (its first lane holds its
+// minimum), and only where the table's value is larger. The top levels use
+// tables indexed by the prefix itself, all filled by the kernel that makes
+// the keys, reduced in shared memory per block. The deeper levels rotate
+// three tables of 8 entries per point; a level's winners reset its entries
+// two kernels later, so the tables are empty again when the build ends.
 //
-// Leaf boxes come from the same per-point enumeration of the nodes (the
-// creator of a level-l node visits it): bottom up, each node's box of leaf
-// cells is the union of its children's, and its record holds its children's
-// boxes quantised outward to 1/256 of a child's edge, the format the render
+// A point's nodes have consecutive ids, each the child of the one before, so
+// spread_kernel writes their child blocks whole and only the first node of a
+// point is linked into its parent (link_kernel).
+//
+// Leaf boxes: climb_kernel starts at every leaf and goes up: a node with one
+// child takes its box shifted; at a node with more, all but the last arriving
+// child's thread stop, and the last, whose siblings' boxes are written by
+// then, makes the union. Each node's record holds its children's boxes
+// quantised outward to 1/256 of a child's edge, the format the render
 // kernels' pruning reads (boxes.cu builds the same records for uploaded
-// trees).
+// trees). No thread waits: a thread that is not last ends.
+//
+// Points given in path order (as assets are) need no creator tables: a point
+// creates the levels below the prefix it shares with the point before it, and
+// the creator of a prefix is the first point of its run, found by a
+// galloping search. A static build, which waits for its node count anyway,
+// looks at the order first.
+//
+// 20M points of a room nearly in path order, 52M nodes: 15 ms of kernels
+// before (the boxes in 12 passes over all points with 64-bit divisions, 7.7
+// ms; node writes out of order 2.5; 13 table passes 2.7; 36 divisions a point
+// for its key 0.5) and 3 ms of allocations; 4.8 ms of kernels now (climb 2.2,
+// bound by its chain of loads; tables 1.7; blocks 0.4; keys 0.3) and 0.4 of
+// allocations. The nodes and records alone are 5.2 GB, 0.8 ms. Boxes by one
+// pass a level without atomics: 3.2 ms instead of the climb's 2.6 then.
 
 #include <cuda_runtime.h>
 #include <thrust/device_vector.h>
 #include <thrust/execution_policy.h>
 #include <thrust/sort.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <vector>
 
@@ -51,26 +70,45 @@ constexpr int kDense = 4;             // levels 1..kDense use prefix-indexed tab
 constexpr int kDenseEntries = 8 + 64 + 512 + 4096;
 constexpr uint64_t kExcluded = ~0ull;  // key of a point left out (bad input)
 constexpr uint32_t kNone = 0xFFFFFFFFu;
+constexpr int kKeyGroups = 4;         // groups of 32 points a warp makes keys of at a time
+constexpr int kClimbThreads = 64;      // threads end at different levels: small blocks give their room back early
 constexpr int kScanThreads = 256, kScanPer = 8, kScanChunk = kScanThreads * kScanPer;
 
 __host__ __device__ constexpr int dense_offset(int l) {  // first entry of level l's prefix table
   return l <= 1 ? 0 : (l == 2 ? 8 : (l == 3 ? 72 : 584));
 }
 
-// Path keys (octets of octree.c:100-109 for points: size halves from the
-// basecube edge, (int)(x / size) % 2 picks the x bit, y and z below the
-// midline set bits 1 and 2; or the given octets), and the per-point state.
-__global__ void keys_kernel(const float* __restrict__ pts, const int32_t* __restrict__ octets, int64_t n,
-                            float basesize, int levels, uint64_t* __restrict__ key, uint8_t* __restrict__ own,
-                            uint32_t* __restrict__ cre, uint32_t* __restrict__ slot, uint32_t* __restrict__ slot_old,
-                            uint32_t* __restrict__ par, unsigned* __restrict__ err) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    uint64_t k = 0;
-    bool ok = true;
-    if (pts) {
-      const float x = pts[3 * i], y = pts[3 * i + 1], z = pts[3 * i + 2];
-      if (!(x >= 0.0f && x < 1.0e30f && y >= 0.0f && y < 1.0e30f && z >= 0.0f && z < 1.0e30f)) {
-        ok = false;
+// The low 21 bits of v, one every third bit.
+__device__ __forceinline__ uint64_t spread3(uint32_t v) {
+  uint64_t x = v & 0x1FFFFFu;
+  x = (x | (x << 32)) & 0x001F00000000FFFFull;
+  x = (x | (x << 16)) & 0x001F0000FF0000FFull;
+  x = (x | (x << 8)) & 0x100F00F00F00F00Full;
+  x = (x | (x << 4)) & 0x10C30C30C30C30C3ull;
+  x = (x | (x << 2)) & 0x1249249249249249ull;
+  return x;
+}
+
+// Path key of point i (octets of octree.c:100-109 for points: size halves
+// from the basecube edge, (int)(x / size) % 2 picks the x bit, y and z below
+// the midline set bits 1 and 2; or the given octets); false for a bad one.
+// Halving is exact for a basecube edge that is far from denormal, so x / size
+// is x / (edge / 2) times a power of two, and the bits of all levels are
+// those of one integer: 3 divisions a point instead of 3 a level.
+__device__ __forceinline__ bool path_key(const float* __restrict__ pts, const int32_t* __restrict__ octets, int64_t i,
+                                         float basesize, int levels, uint64_t* key) {
+  uint64_t k = 0;
+  bool ok = true;
+  if (pts) {
+    const float x = pts[3 * i], y = pts[3 * i + 1], z = pts[3 * i + 2];
+    if (!(x >= 0.0f && x < 1.0e30f && y >= 0.0f && y < 1.0e30f && z >= 0.0f && z < 1.0e30f)) {
+      ok = false;
+    } else if (levels > 0) {
+      const float half = basesize / 2.0f, deep = __int_as_float((126 + levels) << 23);  // 2^(levels - 1)
+      const float qx = (x / half) * deep, qy = (y / half) * deep, qz = (z / half) * deep;
+      if (basesize > 1.0e-20f && fmaxf(fmaxf(qx, qy), qz) < 2147483648.0f) {
+        const uint32_t all = (1u << levels) - 1u;
+        k = spread3((uint32_t)qx & all) | (spread3(~(uint32_t)qy & all) << 1) | (spread3(~(uint32_t)qz & all) << 2);
       } else {
         float size = basesize;
         for (int level = 0; level < levels; ++level) {
@@ -83,100 +121,201 @@ __global__ void keys_kernel(const float* __restrict__ pts, const int32_t* __rest
           k = (k << 3) | (uint64_t)octet;
         }
       }
-    } else {
-      for (int level = 0; level < levels; ++level) {
-        const int o = octets[i * levels + level];
-        ok = ok && o >= 0 && o <= 7;
-        k = (k << 3) | (uint64_t)(o & 7);
-      }
     }
-    if (!ok) atomicOr(err, pts ? kErrBuildPoint : kErrBuildOctet);
-    key[i] = ok ? k : kExcluded;
-    own[i] = (uint8_t)(levels + 1);
-    cre[i] = kNone;  // the root
-    slot[i] = kNone;
-    slot_old[i] = kNone;
-    par[i] = kNone;
+  } else {
+    for (int level = 0; level < levels; ++level) {
+      const int o = octets[i * levels + level];
+      ok = ok && o >= 0 && o <= 7;
+      k = (k << 3) | (uint64_t)(o & 7);
+    }
   }
+  *key = k;
+  return ok;
 }
 
-// Level l: resolve level l - 1 (read the creator of the point's group, note
-// the first level the point creates), reset the level l - 2 table entries,
-// and propose level l (atomicMin of the point index into its group's slot).
-// l runs 1..levels + 1; the last call only resolves.
-__global__ void level_kernel(int l, int levels, int64_t n, const uint64_t* __restrict__ key,
-                             uint8_t* __restrict__ own, uint32_t* __restrict__ cre, uint32_t* __restrict__ slot,
-                             uint32_t* __restrict__ slot_old, uint32_t* __restrict__ par,
-                             const uint32_t* __restrict__ t_res, uint32_t* __restrict__ t_clr,
-                             uint32_t* __restrict__ t_prop, int prop_dense) {
-  extern __shared__ uint32_t sm[];
-  const int entries = prop_dense ? (1 << (3 * l)) : 0;
-  for (int e = threadIdx.x; e < entries; e += blockDim.x) sm[e] = kNone;
-  if (prop_dense) __syncthreads();
-  const int lane = threadIdx.x & 31;
+// Octet of a path key at a level (1..levels).
+__device__ __forceinline__ int key_octet(uint64_t k, int level, int levels) {
+  return (int)(k >> (3 * (levels - level))) & 7;
+}
+
+// min(*t, i) into *t; the atomic only where it would change something (a
+// value read early is never below the current one).
+__device__ __forceinline__ void propose(uint32_t* t, uint32_t i) {
+  if (__ldcg(t) > i) atomicMin(t, i);
+}
+
+// Whether this lane is the first of its run of lanes with equal s (a run's
+// first lane has its smallest point index).
+__device__ __forceinline__ bool run_first(uint32_t s) {
+  const uint32_t before = __shfl_up_sync(0xFFFFFFFFu, s, 1);
+  return (threadIdx.x & 31) == 0 || before != s;
+}
+
+// Path keys, the prefix tables of the top levels (reduced in shared memory
+// per block first), and for a static build whether the points are in path
+// order: own then is the first level each makes, the one after the prefix
+// shared with the point before; *unsorted is set where the order, or a point,
+// is not so (own is then void: first_kernel sets it).
+__global__ void keys_kernel(const float* __restrict__ pts, const int32_t* __restrict__ octets, int64_t n,
+                            float basesize, int levels, uint64_t* __restrict__ key, uint8_t* __restrict__ own,
+                            uint32_t* __restrict__ dense, unsigned* __restrict__ unsorted, unsigned* __restrict__ err) {
+  __shared__ uint32_t sm[kDenseEntries];
+  for (int e = threadIdx.x; e < kDenseEntries; e += blockDim.x) sm[e] = kNone;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, top = levels < kDense ? levels : kDense;
+  bool bad = false;
+  // a warp takes 32 kKeyGroups consecutive points at a time, so that only the
+  // first of them makes the key of the point before it a second time
+  constexpr int kSpan = 32 * kKeyGroups;
+  const int64_t stride = ((int64_t)gridDim.x * blockDim.x >> 5) * kSpan;
+  for (int64_t p0 = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kSpan; p0 < n; p0 += stride) {
+    uint64_t carry = 0;  // key of the point before the group (lane 0)
+    if (unsorted && lane == 0 && p0 > 0) bad |= !path_key(pts, octets, p0 - 1, basesize, levels, &carry);
+#pragma unroll 1
+    for (int g = 0; g < kKeyGroups; ++g) {
+      const int64_t i = p0 + 32 * g + lane;
+      uint64_t k = kExcluded;
+      if (i < n && !path_key(pts, octets, i, basesize, levels, &k)) {
+        k = kExcluded;
+        atomicOr(err, pts ? kErrBuildPoint : kErrBuildOctet);
+      }
+      if (i < n) key[i] = k;
+      if (unsorted) {
+        uint64_t before = __shfl_up_sync(0xFFFFFFFFu, k, 1);
+        if (lane == 0) before = carry;
+        carry = __shfl_sync(0xFFFFFFFFu, k, 31);
+        if (i < n) {
+          bad |= k == kExcluded || (i > 0 && k < before);
+          own[i] = (uint8_t)(i == 0 ? 1
+                             : k == before ? levels + 1
+                                           : levels - (63 - __clzll((long long)(k ^ before))) / 3);
+        }
+      }
+      for (int l = 1; l <= top; ++l) {
+        const uint32_t s = k == kExcluded ? kNone : (uint32_t)(k >> (3 * (levels - l)));
+        const bool first = run_first(s);
+        if (s != kNone && first) {
+          uint32_t* t = sm + dense_offset(l) + s;
+          if (*(volatile uint32_t*)t > (uint32_t)i) atomicMin(t, (uint32_t)i);
+        }
+      }
+    }
+  }
+  if (bad) *unsorted = 1u;
+  __syncthreads();
+  for (int e = threadIdx.x; e < kDenseEntries; e += blockDim.x)
+    if (sm[e] != kNone) propose(dense + e, sm[e]);
+}
+
+// The top levels resolved: the first level each point makes (levels + 1 where
+// none yet), its parent's creator, and the first table level proposed.
+__global__ void first_kernel(int levels, int64_t n, const uint64_t* __restrict__ key, uint8_t* __restrict__ own,
+                             uint32_t* __restrict__ slot, uint32_t* __restrict__ par,
+                             const uint32_t* __restrict__ dense, uint32_t* __restrict__ t_prop) {
+  const int top = levels < kDense ? levels : kDense;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t b0 = (int64_t)blockIdx.x * blockDim.x; b0 < n; b0 += stride) {  // same trip count per block
     const int64_t i = b0 + threadIdx.x;
-    const bool valid = i < n && key[i] != kExcluded;
+    const uint64_t k = i < n ? key[i] : kExcluded;
     uint32_t s = kNone;
-    if (valid) {
-      uint64_t k = key[i];
-      uint32_t c = cre[i];
-      uint32_t so = slot[i];
-      if (l >= 2) {
-        const uint32_t w = t_res[so];
-        if (w == (uint32_t)i && own[i] == (uint8_t)(levels + 1)) {
-          own[i] = (uint8_t)(l - 1);
+    if (k != kExcluded) {
+      uint32_t c = kNone;  // creator of the level's node; the root's: none
+      int o = levels + 1;
+      for (int l = 1; l <= top; ++l) {
+        const uint32_t w = dense[dense_offset(l) + (uint32_t)(k >> (3 * (levels - l)))];
+        if (w == (uint32_t)i && o > levels) {
+          o = l;
           par[i] = c;
         }
         c = w;
-        cre[i] = c;
-        if (t_clr) {
-          const uint32_t sc = slot_old[i];
-          if (sc != kNone) t_clr[sc] = kNone;
-        }
       }
-      if (l <= levels) {
-        const uint64_t prefix = k >> (3 * (levels - l));
-        s = prop_dense ? (uint32_t)prefix : c * 8u + (uint32_t)(prefix & 7u);
-        slot_old[i] = so;
+      own[i] = (uint8_t)o;
+      if (t_prop) {
+        s = c * 8u + (uint32_t)key_octet(k, top + 1, levels);
         slot[i] = s;
       }
+    } else if (i < n) {
+      own[i] = (uint8_t)(levels + 1);
     }
-    if (l <= levels) {
-      if (prop_dense) {
-        if (valid) atomicMin(&sm[s], (uint32_t)i);
-      } else {
-        const unsigned group = __match_any_sync(0xFFFFFFFFu, s);
-        if (valid && lane == __ffs(group) - 1) atomicMin(&t_prop[s], (uint32_t)i);
+    if (t_prop) {
+      const bool first = run_first(s);
+      if (s != kNone && first) propose(t_prop + s, (uint32_t)i);
+    }
+  }
+}
+
+// A point's table slot of a level that it made: its parent's creator is its
+// own index below its first level.
+__device__ __forceinline__ uint32_t made_slot(uint32_t i, int level, int own, const uint32_t* par, uint64_t k,
+                                              int levels) {
+  return (own == level ? par[i] : i) * 8u + (uint32_t)key_octet(k, level, levels);
+}
+
+// Level l > kDense + 1: resolve level l - 1 (a slot's winner is the creator
+// of the group's node; its own slot says its parent's creator), reset the
+// entries of level l - 2 (each by its winner, when every point has read it),
+// and propose level l.
+__global__ void level_kernel(int l, int levels, int64_t n, const uint64_t* __restrict__ key,
+                             uint8_t* __restrict__ own, uint32_t* __restrict__ slot, uint32_t* __restrict__ par,
+                             const uint32_t* __restrict__ t_res, uint32_t* __restrict__ t_clr,
+                             uint32_t* __restrict__ t_prop) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t b0 = (int64_t)blockIdx.x * blockDim.x; b0 < n; b0 += stride) {  // same trip count per block
+    const int64_t i = b0 + threadIdx.x;
+    const uint64_t k = i < n ? key[i] : kExcluded;
+    uint32_t s = kNone;
+    if (k != kExcluded) {
+      const uint32_t so = slot[i];
+      const uint32_t c = t_res[so];
+      int o = own[i];
+      if (c == (uint32_t)i && o > levels) {
+        o = l - 1;
+        own[i] = (uint8_t)o;
+        par[i] = so >> 3;
       }
+      if (t_clr && o <= l - 2) t_clr[made_slot((uint32_t)i, l - 2, o, par, k, levels)] = kNone;
+      s = c * 8u + (uint32_t)key_octet(k, l, levels);
+      slot[i] = s;
     }
-  }
-  if (prop_dense) {
-    __syncthreads();
-    for (int e = threadIdx.x; e < entries; e += blockDim.x)
-      if (sm[e] != kNone) atomicMin(&t_prop[e], sm[e]);
+    const bool first = run_first(s);
+    if (s != kNone && first) propose(t_prop + s, (uint32_t)i);
   }
 }
 
-__device__ __forceinline__ int32_t made(const uint8_t* own, const uint64_t* key, int64_t i, int64_t n, int levels) {
-  if (i >= n || key[i] == kExcluded) return 0;
-  const int o = own[i];
-  return o <= levels ? levels - o + 1 : 0;
+// Nodes point i makes (none for one left out: its first level is past the
+// last).
+__device__ __forceinline__ int32_t made(const uint8_t* own, int64_t i, int64_t n, int levels) {
+  return i < n ? max(levels + 1 - (int)own[i], 0) : 0;
 }
 
-// Prefix sum, pass 1: nodes made per chunk of kScanChunk points; also resets
-// the last level's creator-table entries (all of that level's reads are done).
-__global__ void scan_chunks_kernel(const uint8_t* __restrict__ own, const uint64_t* __restrict__ key, int64_t n,
-                                   int levels, const uint32_t* __restrict__ slot, uint32_t* __restrict__ t_last,
+// Prefix sum, pass 1: nodes made per chunk of kScanChunk points. With
+// creator tables the deepest level is resolved on the way (t_res; and the
+// entries of the level above reset, t_clr), as level_kernel does.
+__global__ void scan_chunks_kernel(uint8_t* __restrict__ own, const uint64_t* __restrict__ key, int64_t n, int levels,
+                                   const uint32_t* __restrict__ slot, uint32_t* __restrict__ par,
+                                   const uint32_t* __restrict__ t_res, uint32_t* __restrict__ t_clr,
                                    int32_t* __restrict__ blocksum) {
   __shared__ int32_t red[kScanThreads];
   const int64_t b = blockIdx.x;
   int32_t sum = 0;
+#pragma unroll
   for (int k = 0; k < kScanPer; ++k) {
-    const int64_t i = b * kScanChunk + (int64_t)threadIdx.x * kScanPer + k;
-    sum += made(own, key, i, n, levels);
-    if (t_last && i < n && key[i] != kExcluded) t_last[slot[i]] = kNone;
+    const int64_t i = b * kScanChunk + (int64_t)k * kScanThreads + threadIdx.x;
+    if (i >= n) break;
+    int o = own[i];
+    if (t_res) {
+      const uint64_t kk = key[i];
+      if (kk != kExcluded) {
+        const uint32_t so = slot[i];
+        if (o > levels && t_res[so] == (uint32_t)i) {
+          o = levels;
+          own[i] = (uint8_t)o;
+          par[i] = so >> 3;
+        }
+        if (t_clr && o <= levels - 1) t_clr[made_slot((uint32_t)i, levels - 1, o, par, kk, levels)] = kNone;
+      }
+    }
+    sum += max(levels + 1 - o, 0);
   }
   red[threadIdx.x] = sum;
   __syncthreads();
@@ -211,125 +350,261 @@ __global__ void scan_top_kernel(int32_t* __restrict__ blocksum, int64_t nb, int3
   if (threadIdx.x == 0) *total = carry;
 }
 
-// Pass 3: each point's first node id; clear the child blocks of the nodes
-// it makes, set their model indices, and give its leaf node the box of its
-// own cell.
-__global__ void scan_nodes_kernel(const uint8_t* __restrict__ own, const uint64_t* __restrict__ key, int64_t n,
-                                  int levels, const int32_t* __restrict__ blocksum, int32_t* __restrict__ base,
-                                  int64_t first_index, int4* __restrict__ child, int32_t* __restrict__ model,
-                                  int32_t* __restrict__ box) {
-  __shared__ int32_t sh[kScanThreads];
-  const int64_t b = blockIdx.x;
-  int32_t mine[kScanPer], sum = 0;
-  for (int k = 0; k < kScanPer; ++k) {
-    mine[k] = made(own, key, b * kScanChunk + (int64_t)threadIdx.x * kScanPer + k, n, levels);
-    sum += mine[k];
+// Pass 3: each point's first node id; the child blocks and model indices of
+// the nodes it makes. A warp takes 32 points at a time; their nodes are one
+// run of ids, and its lanes write that run's blocks (two lanes a block) in
+// order, whichever point a node belongs to.
+__global__ void spread_kernel(const uint8_t* __restrict__ own, const uint64_t* __restrict__ key, int64_t n, int levels,
+                              const int32_t* __restrict__ blocksum, int32_t* __restrict__ base, int64_t first_index,
+                              int4* __restrict__ child, int32_t* __restrict__ model, uint32_t* __restrict__ rec) {
+  constexpr int kWarps = kScanThreads / 32, kGroups = kScanChunk / kScanThreads;
+  __shared__ int32_t sh[kWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t p0 = (int64_t)blockIdx.x * kScanChunk + warp * (kScanChunk / kWarps);
+  int32_t incl[kGroups], sum = 0;
+#pragma unroll
+  for (int g = 0; g < kGroups; ++g) {
+    incl[g] = made(own, p0 + 32 * g + lane, n, levels);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int32_t t = __shfl_up_sync(0xFFFFFFFFu, incl[g], o);
+      if (lane >= o) incl[g] += t;
+    }
+    sum += __shfl_sync(0xFFFFFFFFu, incl[g], 31);
   }
-  sh[threadIdx.x] = sum;
+  if (lane == 0) sh[warp] = sum;
   __syncthreads();
-  for (int o = 1; o < kScanThreads; o <<= 1) {
-    const int32_t t = threadIdx.x >= o ? sh[threadIdx.x - o] : 0;
-    __syncthreads();
-    sh[threadIdx.x] += t;
-    __syncthreads();
-  }
-  int32_t id = blocksum[b] + sh[threadIdx.x] - sum;
-  if (b == 0 && threadIdx.x == 0) {
+  int32_t id = blocksum[blockIdx.x];
+  for (int w = 0; w < warp; ++w) id += sh[w];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    // the root: its links and record come later, where it has children
     child[0] = make_int4(0, 0, 0, 0);
     child[1] = make_int4(0, 0, 0, 0);
     model[0] = 0;
-  }
-  for (int k = 0; k < kScanPer; ++k) {
-    const int64_t i = b * kScanChunk + (int64_t)threadIdx.x * kScanPer + k;
-    if (i >= n) break;
-    base[i] = id;
-    for (int m = 0; m < mine[k]; ++m) {
-      child[2 * (int64_t)(id + m)] = make_int4(0, 0, 0, 0);
-      child[2 * (int64_t)(id + m) + 1] = make_int4(0, 0, 0, 0);
-      model[id + m] = (int32_t)(i + first_index);
-    }
-    if (mine[k] > 0) {
-      int32_t* bx = box + (int64_t)(id + mine[k] - 1) * 6;
-      bx[0] = bx[1] = bx[2] = bx[3] = bx[4] = bx[5] = 0;
-    }
-    id += mine[k];
-  }
-}
-
-// Every made node links itself into its parent.
-__global__ void link_kernel(const uint64_t* __restrict__ key, const uint8_t* __restrict__ own,
-                            const uint32_t* __restrict__ par, const int32_t* __restrict__ base, int64_t n, int levels,
-                            int32_t* __restrict__ child) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t k = key[i];
-    const int o = own[i];
-    if (k == kExcluded || o > levels) continue;
-    const int32_t id0 = base[i];
-    int32_t parent = 0;
-    if (o > 1) {
-      const uint32_t p = par[i];
-      parent = base[p] + (o - 1 - own[p]);
-    }
-    for (int l = o; l <= levels; ++l) {
-      const int32_t id = id0 + (l - o);
-      const int oct = (int)((k >> (3 * (levels - l))) & 7u);
-      child[(int64_t)parent * 8 + oct] = id;
-      parent = id;
-    }
-  }
-}
-
-// Level l's nodes (l < levels): each node's leaf-cell box from its children's
-// (children at level l + 1, done) and its record. The creator of a node
-// visits it; the root is visited by thread 0 of the l = 0 launch.
-__global__ void box_kernel(int l, int levels, const uint64_t* __restrict__ key, const uint8_t* __restrict__ own,
-                           const int32_t* __restrict__ base, int64_t n, const int32_t* __restrict__ child,
-                           int32_t* __restrict__ box, uint32_t* __restrict__ rec) {
-  const int32_t child_cells = 1 << (levels - l - 1);  // leaf cells along a child's edge
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (l == 0 ? 1 : n); i += stride) {
-    int32_t node;
-    if (l == 0) {
-      node = 0;
-    } else {
-      const int o = own[i];
-      if (key[i] == kExcluded || o > l) continue;
-      node = base[i] + (l - o);
-    }
-    int32_t r[6] = {0x7fffffff, -1, 0x7fffffff, -1, 0x7fffffff, -1};
-    uint32_t w[16];
-    const int4* cb4 = reinterpret_cast<const int4*>(child + (int64_t)node * 8);
-    const int4 c0 = cb4[0], c1 = cb4[1];
-    const int32_t ch[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-#pragma unroll
     for (int o = 0; o < 8; ++o) {
-      uint32_t q[6] = {255u, 0u, 255u, 0u, 255u, 0u};  // empty
-      if (ch[o] > 0) {
-        const int32_t* cb = box + (int64_t)ch[o] * 6;
-        if (cb[0] <= cb[1]) {
-          const int32_t off[3] = {(o & 1) ? child_cells : 0, (o & 2) ? child_cells : 0, (o & 4) ? child_cells : 0};
+      rec[2 * o] = 0x00FF00FFu;  // a child without leaves
+      rec[2 * o + 1] = 0x000000FFu;
+    }
+  }
 #pragma unroll
-          for (int a = 0; a < 3; ++a) {
-            r[2 * a] = min(r[2 * a], cb[2 * a] + off[a]);
-            r[2 * a + 1] = max(r[2 * a + 1], cb[2 * a + 1] + off[a]);
-            // [lo, hi + 1) leaf cells in 1/256 of the child's edge, rounded outward
-            const int64_t lo = cb[2 * a], hi1 = (int64_t)cb[2 * a + 1] + 1;
-            const int64_t ql = lo * 256 / child_cells;
-            const int64_t qh = (hi1 * 256 + child_cells - 1) / child_cells - 1;
-            q[2 * a] = (uint32_t)(ql < 0 ? 0 : (ql > 255 ? 255 : ql));
-            q[2 * a + 1] = (uint32_t)(qh < 0 ? 0 : (qh > 255 ? 255 : qh));
+  for (int g = 0; g < kGroups; ++g) {
+    const int64_t i = p0 + 32 * g + lane;
+    const int32_t mine = made(own, i, n, levels);
+    const int32_t total = __shfl_sync(0xFFFFFFFFu, incl[g], 31);
+    const uint64_t k = mine > 0 ? key[i] : 0ull;
+    if (i < n) base[i] = id + incl[g] - mine;
+    for (int32_t j0 = 0; j0 < total; j0 += 16) {
+      const int32_t j = j0 + (lane >> 1);
+      // the point of node j: the first whose nodes end past it
+      int q = 0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        if (__shfl_sync(0xFFFFFFFFu, incl[g], q + o - 1) <= j) q += o;
+      const int32_t end = __shfl_sync(0xFFFFFFFFu, incl[g], q);
+      const uint64_t kq = __shfl_sync(0xFFFFFFFFu, k, q);
+      if (j < total) {
+        const int below = end - 1 - j;  // nodes of the point below this one
+        const int32_t node = id + j;
+        int4 c = make_int4(0, 0, 0, 0);
+        if (below > 0) {
+          const int oct = (int)(kq >> (3 * (below - 1))) & 7;
+          if ((oct >> 2) == (lane & 1)) {
+            c.x = (oct & 3) == 0 ? node + 1 : 0;
+            c.y = (oct & 3) == 1 ? node + 1 : 0;
+            c.z = (oct & 3) == 2 ? node + 1 : 0;
+            c.w = (oct & 3) == 3 ? node + 1 : 0;
           }
         }
+        child[2 * (int64_t)node + (lane & 1)] = c;
+        if (!(lane & 1)) model[node] = (int32_t)(p0 + 32 * g + q + first_index);
       }
-      w[2 * o] = q[0] | (q[1] << 8) | (q[2] << 16) | (q[3] << 24);
-      w[2 * o + 1] = q[4] | (q[5] << 8);
     }
-    int32_t* nb = box + (int64_t)node * 6;
+    id += total;
+  }
+}
+
+// The first node each point makes is linked into its parent, whose id then
+// replaces the parent's creator in par. `sorted`: the creator is not known
+// yet (par is unset): it is the first point of the parent's prefix. maker
+// keeps the creator. t_last: the deepest level's creator table, reset by its
+// winners.
+__global__ void link_kernel(const uint64_t* __restrict__ key, const uint8_t* __restrict__ own,
+                            uint32_t* __restrict__ par, const int32_t* __restrict__ base, int64_t n, int levels,
+                            bool sorted, uint32_t* __restrict__ t_last, int32_t* __restrict__ child,
+                            uint32_t* __restrict__ maker) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int o = own[i];
+    if (o > levels) continue;
+    const uint64_t k = key[i];
+    if (t_last) t_last[made_slot((uint32_t)i, levels, o, par, k, levels)] = kNone;
+    int32_t parent = 0;
+    if (o > 1) {
+      int64_t p;
+      if (sorted) {
+        const int sh = 3 * (levels - o + 1);
+        const uint64_t first = (k >> sh) << sh;
+        // key[lo] < first <= key[hi]; the run starts near i for deep levels
+        int64_t hi = i, step = 1, lo = i - 1;
+        while (lo >= 0 && key[lo] >= first) {
+          hi = lo;
+          step *= 2;
+          lo = hi - step;
+        }
+        if (lo < 0) lo = -1;
+        while (hi - lo > 1) {
+          const int64_t mid = (lo + hi) >> 1;
+          if (key[mid] >= first) hi = mid;
+          else lo = mid;
+        }
+        p = hi;
+      } else {
+        p = par[i];
+      }
+      parent = base[p] + (o - 1 - own[p]);
+      maker[i] = (uint32_t)p;
+    }
+    par[i] = (uint32_t)parent;
+    child[(int64_t)parent * 8 + key_octet(k, o, levels)] = base[i];
+  }
+}
+
+// A box of leaf cells relative to its node: lo x, y, z and hi x, y, z of 21
+// bits each.
+struct CellBox {
+  uint32_t lo[3], hi[3];
+};
+__device__ __forceinline__ uint4 pack_box(const CellBox& b) {
+  const uint64_t l = (uint64_t)b.lo[0] | ((uint64_t)b.lo[1] << 21) | ((uint64_t)b.lo[2] << 42);
+  const uint64_t h = (uint64_t)b.hi[0] | ((uint64_t)b.hi[1] << 21) | ((uint64_t)b.hi[2] << 42);
+  return make_uint4((uint32_t)l, (uint32_t)(l >> 32), (uint32_t)h, (uint32_t)(h >> 32));
+}
+__device__ __forceinline__ CellBox unpack_box(uint4 v) {
+  const uint64_t l = (uint64_t)v.x | ((uint64_t)v.y << 32), h = (uint64_t)v.z | ((uint64_t)v.w << 32);
+  CellBox b;
 #pragma unroll
-    for (int a = 0; a < 6; ++a) nb[a] = r[a];
-    uint4* dst = reinterpret_cast<uint4*>(rec + (int64_t)node * 16);
+  for (int a = 0; a < 3; ++a) {
+    b.lo[a] = (uint32_t)(l >> (21 * a)) & 0x1FFFFFu;
+    b.hi[a] = (uint32_t)(h >> (21 * a)) & 0x1FFFFFu;
+  }
+  return b;
+}
+
+// Record word of a child of 2^sh leaf cells an edge with box b: [lo, hi + 1)
+// in 1/256 of the edge, rounded outward.
+__device__ __forceinline__ uint2 record_word(const CellBox& b, int sh) {
+  uint32_t q[6];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) dst[k] = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
+  for (int a = 0; a < 3; ++a) {
+    const uint32_t lo = b.lo[a], hi1 = b.hi[a] + 1u;
+    q[2 * a] = sh >= 8 ? lo >> (sh - 8) : lo << (8 - sh);
+    q[2 * a + 1] = (sh >= 8 ? (hi1 + (1u << (sh - 8)) - 1u) >> (sh - 8) : hi1 << (8 - sh)) - 1u;
+  }
+  return make_uint2(q[0] | (q[1] << 8) | (q[2] << 16) | (q[3] << 24), q[4] | (q[5] << 8));
+}
+
+// Union of the boxes of a node's children (2^sh leaf cells an edge) into b,
+// and the node's record.
+__device__ __forceinline__ void join_boxes(const int32_t (&ch)[8], const uint4* box, int sh, CellBox& b,
+                                           uint32_t (&w)[16]) {
+  b = {{0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, {0u, 0u, 0u}};
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    w[2 * q] = 0x00FF00FFu;  // a child without leaves
+    w[2 * q + 1] = 0x000000FFu;
+    if (ch[q] <= 0) continue;
+    const CellBox c = unpack_box(__ldcg(box + ch[q]));
+    const uint2 r = record_word(c, sh);
+    w[2 * q] = r.x;
+    w[2 * q + 1] = r.y;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const uint32_t off = ((q >> a) & 1) ? 1u << sh : 0u;
+      b.lo[a] = min(b.lo[a], c.lo[a] + off);
+      b.hi[a] = max(b.hi[a], c.hi[a] + off);
+    }
+  }
+}
+
+// A node's child block, and its record, by 32-byte accesses (whole sectors).
+__device__ __forceinline__ void load_children(const int4* __restrict__ child, int32_t node, int32_t (&ch)[8]) {
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(ch[0]), "=r"(ch[1]), "=r"(ch[2]), "=r"(ch[3]), "=r"(ch[4]), "=r"(ch[5]), "=r"(ch[6]), "=r"(ch[7])
+               : "l"(child + 2 * (int64_t)node));
+}
+
+__device__ __forceinline__ void store_record(uint4* __restrict__ rec, int32_t node, const uint32_t (&w)[16]) {
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(rec + (int64_t)node * 4 + 2 * q),
+                 "r"(w[8 * q]), "r"(w[8 * q + 1]), "r"(w[8 * q + 2]), "r"(w[8 * q + 3]), "r"(w[8 * q + 4]),
+                 "r"(w[8 * q + 5]), "r"(w[8 * q + 6]), "r"(w[8 * q + 7])
+                 : "memory");
+}
+
+// Leaf boxes, from every leaf up (see the top). par holds the parent node of
+// each point's first node; arrived 4 bits a node, zero.
+__global__ void __launch_bounds__(kClimbThreads, 24) climb_kernel(const uint64_t* __restrict__ key, const uint8_t* __restrict__ own,
+                             const uint32_t* __restrict__ par, const int32_t* __restrict__ base, int64_t n, int levels,
+                             const uint32_t* __restrict__ maker, const int4* __restrict__ child, uint4* box,
+                             uint32_t* arrived, uint4* __restrict__ rec) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  int o = own[i];
+  if (o > levels) return;
+  const uint64_t k = key[i];
+  int32_t node = base[i] + (levels - o);
+  uint32_t p = (uint32_t)i;  // the point whose nodes the climb is among
+  CellBox b = {{0u, 0u, 0u}, {0u, 0u, 0u}};
+  for (int l = levels - 1; l >= 0; --l) {
+    int32_t parent = node - 1;
+    if (l + 1 == o) {
+      parent = (int32_t)par[p];
+      if (l > 0) {
+        p = maker[p];
+        o = own[p];
+      }
+    }
+    const int sh = levels - 1 - l;
+    const int oct = key_octet(k, l + 1, levels);
+    int32_t ch[8];
+    load_children(child, parent, ch);
+    int count = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) count += ch[q] > 0 ? 1 : 0;
+    uint32_t w[16];
+    if (count == 1) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        w[2 * q] = 0x00FF00FFu;
+        w[2 * q + 1] = 0x000000FFu;
+      }
+      const uint2 r = record_word(b, sh);
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (q == oct) {
+          w[2 * q] = r.x;
+          w[2 * q + 1] = r.y;
+        }
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const uint32_t off = ((oct >> a) & 1) ? 1u << sh : 0u;
+        b.lo[a] += off;
+        b.hi[a] += off;
+      }
+    } else {
+      // the arrival releases this child's box and acquires its siblings'
+      __stcg(box + node, pack_box(b));
+      const uint32_t at = 4u * ((uint32_t)parent & 7u);
+      uint32_t before;
+      asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;"
+                   : "=r"(before)
+                   : "l"(arrived + ((uint32_t)parent >> 3)), "r"(1u << at)
+                   : "memory");
+      if ((int)((before >> at) & 15u) != count - 1) return;
+      join_boxes(ch, box, sh, b, w);
+    }
+    store_record(rec, parent, w);
+    node = parent;
   }
 }
 
@@ -361,48 +636,53 @@ int64_t build_node_bound(int64_t n, int levels) {
 }
 
 void build_release(BuildScratch* s) {
-  void* ptrs[] = {s->key, s->cre, s->slot, s->slot_old, s->par, s->base, s->own, s->tab[0], s->tab[1], s->tab[2],
-                  s->dense, s->blocksum, s->box};
+  void* ptrs[] = {s->key, s->slot, s->par, s->base, s->own, s->tab[0], s->tab[1], s->tab[2],
+                  s->dense, s->blocksum, s->box, s->arrived};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   *s = BuildScratch();
 }
 
-int build_reserve(BuildScratch* s, int64_t n, int levels) {
+int build_check(int64_t n, int levels) {
   if (n > ((int64_t)1 << 29)) return fail(QBC_E_ARG, "tree build: %lld points exceed 2^29", (long long)n);
   const int64_t nodes = build_node_bound(n, levels);
   if (nodes > INT32_MAX) return fail(QBC_E_ARG, "tree build: up to %lld nodes exceed int32 indices", (long long)nodes);
-  int rc = QBC_OK;
+  return QBC_OK;
+}
+
+int build_reserve(BuildScratch* s, int64_t n, int levels) {
+  int rc = build_check(n, levels);
+  if (rc) return rc;
+  const int64_t nodes = build_node_bound(n, levels);
+  const int64_t m = std::max<int64_t>(n, 1);
   if (s->points < n || !s->key) {
-    const int64_t m = std::max<int64_t>(n, 1);
+    s->points = 0;
     if (!rc) rc = grow_buf(&s->key, 0, m, "keys");
-    if (!rc) rc = grow_buf(&s->cre, 0, m, "creators");
-    if (!rc) rc = grow_buf(&s->slot, 0, m, "slots");
-    if (!rc) rc = grow_buf(&s->slot_old, 0, m, "slots");
     if (!rc) rc = grow_buf(&s->par, 0, m, "parents");
     if (!rc) rc = grow_buf(&s->base, 0, m, "node ids");
     if (!rc) rc = grow_buf(&s->own, 0, m, "levels");
+    if (!rc) rc = grow_buf(&s->slot, 0, m, "slots");
     if (rc) return rc;
     s->points = m;
   }
   if (levels > kDense && (s->tab_points < n || !s->tab[0])) {
-    const int64_t m = std::max<int64_t>(n, 1);
+    s->tab_points = 0;
     for (int t = 0; t < 3 && !rc; ++t) rc = grow_buf(&s->tab[t], 0, 8 * m, "creator tables");
     if (rc) return rc;
-    for (int t = 0; t < 3; ++t) {
-      cudaError_t e = cudaMemset(s->tab[t], 0xFF, (size_t)8 * m * sizeof(uint32_t));
-      if (e != cudaSuccess) return fail(QBC_E_CUDA, "tree build: clear creator tables: %s", cudaGetErrorString(e));
-    }
     s->tab_points = m;
+    s->dirty = true;  // emptied on the build's stream
   }
   const int64_t nb = (n + kScanChunk - 1) / kScanChunk;
   if (s->blocks < nb || !s->blocksum) {
+    s->blocks = 0;
     rc = grow_buf(&s->blocksum, 0, std::max<int64_t>(nb, 1), "block sums");
     if (rc) return rc;
     s->blocks = std::max<int64_t>(nb, 1);
   }
   if (s->box_nodes < nodes || !s->box) {
-    rc = grow_buf(&s->box, 0, 6 * nodes, "leaf boxes");
+    s->box_nodes = 0;
+    rc = grow_buf(&s->box, 0, nodes, "leaf boxes");
+    if (!rc) rc = grow_buf(&s->arrived, 0, nodes / 8 + 1, "arrivals");
     if (rc) return rc;
     s->box_nodes = nodes;
   }
@@ -410,55 +690,96 @@ int build_reserve(BuildScratch* s, int64_t n, int levels) {
   return rc;
 }
 
+namespace {
+
+// Creator table of a level past the prefix tables.
+uint32_t* level_table(const BuildScratch* s, int l) { return s->tab[l % 3]; }
+
+// Ids by a prefix sum, once each point's first level (and, unless sorted,
+// its parent's creator; with tables, but for the deepest level) is known. The
+// node count goes to *total.
+void count_nodes(int64_t n, int levels, const BuildScratch* s, bool sorted, int32_t* total, cudaStream_t stream,
+                 int64_t* launches) {
+  const int64_t nb = std::max<int64_t>(1, (n + kScanChunk - 1) / kScanChunk);
+  const bool tables = !sorted && levels > kDense;
+  scan_chunks_kernel<<<(unsigned)nb, kScanThreads, 0, stream>>>(
+      s->own, s->key, n, levels, s->slot, s->par, tables ? level_table(s, levels) : nullptr,
+      tables && levels - 1 > kDense ? level_table(s, levels - 1) : nullptr, s->blocksum);
+  scan_top_kernel<<<1, 1024, 0, stream>>>(s->blocksum, nb, total);
+  *launches += 2;
+}
+
+// Blocks, links and boxes of at most `nodes` nodes. reset: leave the creator
+// tables empty for the next build.
+void write_tree(int64_t n, int levels, int64_t first_index, const BuildScratch* s, bool sorted, bool reset,
+                int64_t nodes, int32_t* child, int32_t* model, uint32_t* rec, cudaStream_t stream,
+                int64_t* launches) {
+  const int64_t nb = std::max<int64_t>(1, (n + kScanChunk - 1) / kScanChunk);
+  spread_kernel<<<(unsigned)nb, kScanThreads, 0, stream>>>(s->own, s->key, n, levels, s->blocksum, s->base,
+                                                           first_index, reinterpret_cast<int4*>(child), model, rec);
+  ++*launches;
+  if (n > 0 && levels > 0) {
+    const int4* blocks = reinterpret_cast<const int4*>(child);
+    uint4* records = reinterpret_cast<uint4*>(rec);
+    // (the slots are done: their array takes the parents' creators)
+    link_kernel<<<grid_for(n), 256, 0, stream>>>(s->key, s->own, s->par, s->base, n, levels, sorted,
+                                                 reset && levels > kDense ? level_table(s, levels) : nullptr, child,
+                                                 s->slot);
+    ++*launches;
+    cudaMemsetAsync(s->arrived, 0, (size_t)(nodes / 8 + 1) * sizeof(uint32_t), stream);
+    climb_kernel<<<(unsigned)((n + kClimbThreads - 1) / kClimbThreads), kClimbThreads, 0, stream>>>(
+        s->key, s->own, s->par, s->base, n, levels, s->slot, blocks, s->box, s->arrived, records);
+    ++*launches;
+  }
+}
+
+int keys_and_prefixes(const float* d_pts, const int32_t* d_octets, int64_t n, float basesize, int levels,
+                      BuildScratch* s, unsigned* unsorted, unsigned* err, cudaStream_t stream, int grid,
+                      int64_t* launches) {
+  if (levels < 0 || levels > kMaxBuildLevels) return fail(QBC_E_ARG, "tree build: levels %d outside 0..21", levels);
+  if (n < 0 || n > s->points) return fail(QBC_E_ARG, "tree build: %lld points beyond the reserved scratch", (long long)n);
+  if (cudaMemsetAsync(s->dense, 0xFF, kDenseEntries * sizeof(uint32_t), stream) != cudaSuccess)
+    return fail(QBC_E_CUDA, "tree build: reset prefix tables");
+  if (n > 0) {
+    keys_kernel<<<std::max(1, std::min(grid, grid_for(n))), 256, 0, stream>>>(d_pts, d_octets, n, basesize, levels,
+                                                                              s->key, s->own, s->dense, unsorted, err);
+    ++*launches;
+  }
+  return QBC_OK;
+}
+
+// After keys_and_prefixes: creators by table (the deepest level's are left to
+// count_nodes).
+void table_levels(int64_t n, int levels, const BuildScratch* s, cudaStream_t stream, int grid, int64_t* launches) {
+  if (n <= 0) return;
+  const int g = std::max(1, std::min(grid, grid_for(n)));
+  first_kernel<<<g, 256, 0, stream>>>(levels, n, s->key, s->own, s->slot, s->par, s->dense,
+                                      levels > kDense ? level_table(s, kDense + 1) : nullptr);
+  ++*launches;
+  for (int l = kDense + 2; l <= levels; ++l) {
+    level_kernel<<<g, 256, 0, stream>>>(l, levels, n, s->key, s->own, s->slot, s->par, level_table(s, l - 1),
+                                        l - 2 > kDense ? level_table(s, l - 2) : nullptr, level_table(s, l));
+    ++*launches;
+  }
+}
+
+}  // namespace
+
 int build_tree_async(const float* d_pts, const int32_t* d_octets, int64_t n, float basesize, int levels,
                      int64_t first_index, BuildScratch* s, int32_t* child, int32_t* model, uint32_t* rec,
                      int32_t* total, unsigned* err, cudaStream_t stream, int grid, int64_t* launches) {
-  if (levels < 0 || levels > kMaxBuildLevels) return fail(QBC_E_ARG, "tree build: levels %d outside 0..21", levels);
-  if (n < 0 || n > s->points) return fail(QBC_E_ARG, "tree build: %lld points beyond the reserved scratch", (long long)n);
+  const int64_t L0 = *launches;
+  int rc = keys_and_prefixes(d_pts, d_octets, n, basesize, levels, s, nullptr, err, stream, grid, launches);
+  if (rc) return rc;
   if (levels > kDense && s->dirty) {
     for (int t = 0; t < 3; ++t)
       if (cudaMemsetAsync(s->tab[t], 0xFF, (size_t)8 * s->tab_points * sizeof(uint32_t), stream) != cudaSuccess)
         return fail(QBC_E_CUDA, "tree build: reset creator tables");
   }
   s->dirty = true;
-  int64_t L0 = *launches;
-  const int g = std::max(1, std::min(grid, grid_for(n)));
-  if (cudaMemsetAsync(s->dense, 0xFF, kDenseEntries * sizeof(uint32_t), stream) != cudaSuccess)
-    return fail(QBC_E_CUDA, "tree build: reset prefix tables");
-  if (n > 0)
-    keys_kernel<<<g, 256, 0, stream>>>(d_pts, d_octets, n, basesize, levels, s->key, s->own, s->cre, s->slot,
-                                       s->slot_old, s->par, err);
-  ++*launches;
-  auto table = [&](int l) -> uint32_t* {
-    return l <= kDense ? s->dense + dense_offset(l) : s->tab[l % 3];
-  };
-  for (int l = 1; l <= levels + 1 && n > 0; ++l) {
-    const bool pd = l <= levels && l <= kDense;
-    const uint32_t* t_res = l >= 2 ? table(l - 1) : nullptr;
-    uint32_t* t_clr = (l >= 3 && l - 2 > kDense) ? table(l - 2) : nullptr;
-    uint32_t* t_prop = l <= levels ? table(l) : nullptr;
-    const size_t smem = pd ? sizeof(uint32_t) << (3 * l) : 0;
-    level_kernel<<<g, 256, smem, stream>>>(l, levels, n, s->key, s->own, s->cre, s->slot, s->slot_old, s->par, t_res,
-                                           t_clr, t_prop, pd ? 1 : 0);
-    ++*launches;
-  }
-  const int64_t nb = std::max<int64_t>(1, (n + kScanChunk - 1) / kScanChunk);
-  scan_chunks_kernel<<<(unsigned)nb, kScanThreads, 0, stream>>>(s->own, s->key, n, levels, s->slot,
-                                                                 levels > kDense ? table(levels) : nullptr,
-                                                                 s->blocksum);
-  scan_top_kernel<<<1, 1024, 0, stream>>>(s->blocksum, nb, total);
-  scan_nodes_kernel<<<(unsigned)nb, kScanThreads, 0, stream>>>(s->own, s->key, n, levels, s->blocksum, s->base,
-                                                                first_index, reinterpret_cast<int4*>(child), model,
-                                                                s->box);
-  *launches += 3;
-  if (n > 0) {
-    link_kernel<<<g, 256, 0, stream>>>(s->key, s->own, s->par, s->base, n, levels, child);
-    ++*launches;
-  }
-  for (int l = levels - 1; l >= 0; --l) {
-    box_kernel<<<l == 0 ? 1 : g, 256, 0, stream>>>(l, levels, s->key, s->own, s->base, n, child, s->box, rec);
-    ++*launches;
-  }
+  table_levels(n, levels, s, stream, grid, launches);
+  count_nodes(n, levels, s, false, total, stream, launches);
+  write_tree(n, levels, first_index, s, false, true, build_node_bound(n, levels), child, model, rec, stream, launches);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     *launches = L0;
@@ -466,6 +787,96 @@ int build_tree_async(const float* d_pts, const int32_t* d_octets, int64_t n, flo
   }
   s->dirty = false;
   return QBC_OK;
+}
+
+namespace {
+
+// Device memory of one build, freed when the stream is done with it.
+struct Arena {
+  cudaStream_t stream;
+  std::vector<void*> held;
+  explicit Arena(cudaStream_t s) : stream(s) {}
+  ~Arena() {
+    cudaStreamSynchronize(stream);
+    for (void* p : held) cudaFree(p);
+  }
+  void* take(size_t bytes) {
+    void* p = nullptr;
+    if (cudaMalloc(&p, std::max<size_t>(bytes, 256)) != cudaSuccess) return nullptr;
+    held.push_back(p);
+    return p;
+  }
+};
+
+}  // namespace
+
+int build_tree_static(const float* d_pts, const int32_t* d_octets, int64_t n, float basesize, int levels,
+                      int64_t first_index, int32_t* child, int32_t* model, uint32_t* rec, int64_t rec_nodes,
+                      int32_t* d_total, int64_t* total, unsigned* flag, unsigned* err, cudaStream_t stream, int grid,
+                      int64_t* launches) {
+  BuildScratch s;
+  Arena arena(stream);
+  // per-point state in one allocation, its parts 256-byte aligned
+  const int64_t m = std::max<int64_t>(n, 1), nb = std::max<int64_t>((n + kScanChunk - 1) / kScanChunk, 1);
+  size_t off = 0;
+  auto part = [&](size_t bytes) {
+    const size_t at = off;
+    off += (bytes + 255) & ~size_t(255);
+    return at;
+  };
+  const size_t key = part(8 * m), par = part(4 * m), base = part(4 * m), own = part(m), slot = part(4 * m),
+               sums = part(4 * nb), dense = part(4 * kDenseEntries);
+  char* p = static_cast<char*>(arena.take(off));
+  if (!p) return fail(QBC_E_NOMEM, "tree build: scratch of %zu bytes", off);
+  s.points = n;
+  s.key = reinterpret_cast<uint64_t*>(p + key);
+  s.par = reinterpret_cast<uint32_t*>(p + par);
+  s.base = reinterpret_cast<int32_t*>(p + base);
+  s.own = reinterpret_cast<uint8_t*>(p + own);
+  s.slot = reinterpret_cast<uint32_t*>(p + slot);
+  s.blocksum = reinterpret_cast<int32_t*>(p + sums);
+  s.dense = reinterpret_cast<uint32_t*>(p + dense);
+
+  unsigned unsorted = levels > 0 ? 0u : 1u;
+  cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(unsigned), stream);
+  if (e != cudaSuccess) return fail(QBC_E_CUDA, "tree build: %s", cudaGetErrorString(e));
+  int rc = keys_and_prefixes(d_pts, d_octets, n, basesize, levels, &s, levels > 0 ? flag : nullptr, err, stream, grid,
+                         launches);
+  if (rc) return rc;
+  if (levels > 0) {
+    e = cudaMemcpyAsync(&unsorted, flag, sizeof(unsigned), cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    if (e != cudaSuccess) return fail(QBC_E_CUDA, "tree build: %s", cudaGetErrorString(e));
+  }
+  if (unsorted) {
+    if (levels > kDense) {
+      // the tables lie where the records will be, unless there are too few
+      const size_t each = (size_t)32 * m, all = 3 * each;
+      char* t = reinterpret_cast<char*>(rec);
+      if (all > (size_t)rec_nodes * 64) t = static_cast<char*>(arena.take(all));
+      if (!t) return fail(QBC_E_NOMEM, "tree build: creator tables of %zu bytes", all);
+      for (int k = 0; k < 3; ++k) s.tab[k] = reinterpret_cast<uint32_t*>(t + k * each);
+      e = cudaMemsetAsync(t, 0xFF, all, stream);
+      if (e != cudaSuccess) return fail(QBC_E_CUDA, "tree build: %s", cudaGetErrorString(e));
+    }
+    table_levels(n, levels, &s, stream, grid, launches);
+  }
+  count_nodes(n, levels, &s, !unsorted, d_total, stream, launches);
+  int32_t h = 0;
+  e = cudaMemcpyAsync(&h, d_total, sizeof(h), cudaMemcpyDeviceToHost, stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+  if (e != cudaSuccess) return fail(QBC_E_CUDA, "tree build: %s", cudaGetErrorString(e));
+  *total = h;
+  // exact boxes and arrival counts past the records, where they fit
+  const size_t boxes = (size_t)h * 16, counts = ((size_t)h / 8 + 1) * 4, used = (size_t)h * 64;
+  char* t = reinterpret_cast<char*>(rec) + used;
+  if (used + boxes + counts > (size_t)rec_nodes * 64) t = static_cast<char*>(arena.take(boxes + counts));
+  if (!t) return fail(QBC_E_NOMEM, "tree build: leaf boxes of %zu bytes", boxes + counts);
+  s.box = reinterpret_cast<uint4*>(t);
+  s.arrived = reinterpret_cast<uint32_t*>(t + boxes);
+  write_tree(n, levels, first_index, &s, !unsorted, false, h, child, model, rec, stream, launches);
+  e = cudaGetLastError();
+  return e == cudaSuccess ? QBC_OK : fail(QBC_E_CUDA, "tree build: %s", cudaGetErrorString(e));
 }
 
 namespace {

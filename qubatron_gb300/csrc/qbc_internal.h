@@ -29,31 +29,33 @@ enum DeviceError : unsigned {
   kErrRecordOverflow = 16u,  // a split frame's record queue was full (pixels left unwritten)
 };
 
-// Scratch of the GPU tree build, owned by the context and reused by every
-// build: it grows to the largest build seen, so repeated builds of up to that
+// Scratch of the dynamic tree's GPU build, owned by the context and reused by
+// every build: it grows to the largest build seen, so repeated builds of up to that
 // size allocate nothing.
 struct BuildScratch {
-  int64_t points = 0;        // per-point arrays hold this many points
+  int64_t points = 0;        // the per-point arrays hold this many points
   int64_t tab_points = 0;    // creator tables hold 8 entries per point for this many
   int64_t blocks = 0;        // prefix-sum block sums
-  int64_t box_nodes = 0;     // exact leaf-cell boxes (6 int32 per node)
+  int64_t box_nodes = 0;     // exact leaf-cell boxes and arrival counts hold this many nodes
   uint64_t* key = nullptr;   // path key, 3 bits per level, root level most significant
-  uint32_t* cre = nullptr;   // creator of the point's node at the last resolved level
-  uint32_t* slot = nullptr;  // table slot of the last proposed level
-  uint32_t* slot_old = nullptr;  // table slot of the level before it
-  uint32_t* par = nullptr;   // creator of the parent of the point's first own node
+  uint32_t* slot = nullptr;  // table slot of the last proposed level, then the creator of par
+  uint32_t* par = nullptr;   // creator of the parent of the point's first own node, then the parent's id
   int32_t* base = nullptr;   // id of the point's first own node
   uint8_t* own = nullptr;    // first level whose node the point creates (levels + 1: none)
   uint32_t* tab[3] = {nullptr, nullptr, nullptr};  // creator tables of the deeper levels
   uint32_t* dense = nullptr;  // prefix tables of the top levels
   int32_t* blocksum = nullptr;
-  int32_t* box = nullptr;
-  bool dirty = false;        // a build stopped midway: tables must be reset
+  uint4* box = nullptr;      // boxes of nodes with siblings, 6 x 21 bits
+  uint32_t* arrived = nullptr;  // children done, 4 bits a node
+  bool dirty = false;        // tables new, or left by a build that stopped midway: to be emptied
 };
 
 // Nodes a build of n points at `levels` can make: 1 + sum over levels l of
 // min(n, 8^l).
 int64_t build_node_bound(int64_t n, int levels);
+
+// Whether a build of this size can be numbered.
+int build_check(int64_t n, int levels);
 
 // Grow the scratch for n points at `levels` (allocates only when it grows).
 int build_reserve(BuildScratch* s, int64_t n, int levels);
@@ -71,6 +73,17 @@ void build_release(BuildScratch* s);
 int build_tree_async(const float* d_pts, const int32_t* d_octets, int64_t n, float basesize, int levels,
                      int64_t first_index, BuildScratch* s, int32_t* child, int32_t* model, uint32_t* rec,
                      int32_t* total, unsigned* err, cudaStream_t stream, int grid, int64_t* launches);
+
+// The same for a build that may wait (two host synchronisations), with
+// scratch of its own, freed at the end: 21 bytes a point. It looks whether the
+// points are in path order (`flag`: a device word) and then does without the
+// creator tables; the tables, and later the exact boxes, lie in the space of
+// rec (rec_nodes records) that holds no records yet, or else are allocated.
+// The node count goes to *total (d_total: a device word).
+int build_tree_static(const float* d_pts, const int32_t* d_octets, int64_t n, float basesize, int levels,
+                      int64_t first_index, int32_t* child, int32_t* model, uint32_t* rec, int64_t rec_nodes,
+                      int32_t* d_total, int64_t* total, unsigned* flag, unsigned* err, cudaStream_t stream, int grid,
+                      int64_t* launches);
 
 // octree_remove_point (octree.c:182-218) of n points in order, on a device
 // tree (child: 8 int32 per node, model: 1 per node): cuts the links in place,

@@ -509,9 +509,9 @@ int stage_build_input(qbc_ctx* c, const float* pnts, const int32_t* octets, int6
 // A GPU build into tree `tree` (qbc_build_tree, qbc_build_tree_paths,
 // qbc_load_flat). Buffers are sized for the build's node bound, so a build of
 // the same size as the last one allocates nothing, and nothing is read back:
-// the exact node count stays on the device. A static-tree build frees the
-// build scratch afterwards (a one-time build); a dynamic-tree build keeps it
-// for the next frame.
+// the exact node count stays on the device. A static-tree build waits for its
+// count and has scratch of its own (a one-time build); a dynamic-tree build
+// keeps its scratch with the context for the next frame.
 int build_into(qbc_ctx* c, int tree, const float* pnts, const int32_t* octets, int64_t n, float basesize, int levels,
                int64_t first_index, int on_device) {
   if (!c || tree < 0 || tree > 1) return fail(QBC_E_ARG, "tree build: bad context or tree id");
@@ -520,16 +520,16 @@ int build_into(qbc_ctx* c, int tree, const float* pnts, const int32_t* octets, i
   if (levels < 0 || levels > 21) return fail(QBC_E_ARG, "tree build: levels %d outside 0..21", levels);
   QBC_CUDA(cudaSetDevice(c->device));
   const void* dev = pnts ? (const void*)pnts : (const void*)octets;
-  if (!on_device && n > 0) {
-    int rc = stage_build_input(c, pnts, octets, n, levels, &dev);
-    if (rc) return rc;
-  }
-  int rc = qbc::build_reserve(&c->build, n, levels);
+  int rc = QBC_OK;
+  if (!on_device && n > 0 && (rc = stage_build_input(c, pnts, octets, n, levels, &dev))) return rc;
+  rc = tree == 0 ? qbc::build_check(n, levels) : qbc::build_reserve(&c->build, n, levels);
   if (rc) return rc;
   DevTreeBuf& tb = c->tree[tree];
   const int64_t bound = qbc::build_node_bound(n, levels);
   if (tb.cap < bound || !tb.child) {
     int64_t cap = 0;
+    tb.n = 0;  // what the buffers held goes
+    tb.count_on_device = false;
     rc = grow(&tb.child, &cap, bound, 32, "octree child blocks");
     if (!rc) rc = grow(&tb.model, &tb.cap, bound, 4, "octree model indices");
     if (rc) return rc;
@@ -538,27 +538,31 @@ int build_into(qbc_ctx* c, int tree, const float* pnts, const int32_t* octets, i
     rc = grow(&tb.cbox, &tb.cbox_cap, bound, 64, "octree leaf boxes");
     if (rc) return rc;
   }
-  rc = qbc::build_tree_async(pnts ? static_cast<const float*>(dev) : nullptr,
-                             pnts ? nullptr : static_cast<const int32_t*>(dev), n, basesize, levels, first_index,
-                             &c->build, reinterpret_cast<int32_t*>(tb.child), tb.model, tb.cbox, tb.d_count, c->derr,
-                             c->stream, c->sm_count * 8, &c->launches);
-  if (rc) return rc;
-  tb.n = bound;
-  tb.count_on_device = true;
-  tb.box_depth = levels <= QBC_MAX_LEVEL ? levels : -1;
-  tb.box_valid = true;
+  const float* dp = pnts ? static_cast<const float*>(dev) : nullptr;
+  const int32_t* dq = pnts ? nullptr : static_cast<const int32_t*>(dev);
+  int32_t* child = reinterpret_cast<int32_t*>(tb.child);
+  const int grid = c->sm_count * 8;
+  tb.box_valid = false;  // (until the build stands: its scratch may lie in the records)
   if (tree == 0) {
     // a one-time build: the exact count bounds the kernels' index checks
     int64_t exact = 0;
-    rc = tree_count(c, 0, &exact);
+    rc = qbc::build_tree_static(dp, dq, n, basesize, levels, first_index, child, tb.model, tb.cbox, tb.cbox_cap,
+                                tb.d_count, &exact, c->queue, c->derr, c->stream, grid, &c->launches);
     if (rc) return rc;
     tb.n = exact;
     tb.count_on_device = false;
-    qbc::build_release(&c->build);
-    cudaFree(c->build_input);
+    if (c->build_input) cudaFree(c->build_input);
     c->build_input = nullptr;
     c->build_input_cap = 0;
+  } else {
+    rc = qbc::build_tree_async(dp, dq, n, basesize, levels, first_index, &c->build, child, tb.model, tb.cbox,
+                               tb.d_count, c->derr, c->stream, grid, &c->launches);
+    if (rc) return rc;
+    tb.n = bound;
+    tb.count_on_device = true;
   }
+  tb.box_depth = levels <= QBC_MAX_LEVEL ? levels : -1;
+  tb.box_valid = true;
   return QBC_OK;
 }
 

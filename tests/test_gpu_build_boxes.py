@@ -1,0 +1,53 @@
+"""Trees built on the GPU, from points in path order (no creator tables) and
+from shuffled ones, at the sizes where a warp's, a block's or a chunk's points
+end: node arrays equal the host producer's, and the leaf boxes equal those
+built for the same array uploaded: every ray's visit count depends on them."""
+import numpy as np
+import pytest
+
+from conftest import S
+
+pytestmark = pytest.mark.gpu
+
+
+def _points(n, levels, rng, order):
+    # clusters with duplicates, so that chains, branches and equal cells occur
+    c = rng.uniform(0.0, S, (max(n // 20, 1), 3))
+    p = c[rng.integers(0, c.shape[0], n)] + rng.normal(size=(n, 3)) * S * rng.choice([0.0, 1e-3, 0.1], (n, 1))
+    p = np.clip(p, 0.0, np.nextafter(np.float32(S), np.float32(0.0))).astype(np.float32)
+    if order == "shuffled":
+        return p
+    from oracle import qbo
+    o = qbo.point_octets(p, S, levels).astype(np.int64)
+    key = np.zeros(n, np.int64)
+    for k in range(levels):
+        key = key * 8 + o[:, k]
+    idx = np.argsort(key, kind="stable")
+    if order == "one out":  # in path order but for one point
+        idx[[0, n // 2]] = idx[[n // 2, 0]]
+    return p[idx]
+
+
+@pytest.mark.parametrize("order", ["sorted", "one out", "shuffled"])
+@pytest.mark.parametrize("n,levels", [(1, 1), (1, 17), (2, 3), (31, 12), (32, 5), (33, 12), (2047, 12), (2048, 9),
+                                      (2049, 16), (6000, 2), (6000, 12), (20000, 17), (3000, 21)])
+def test_built_tree_and_boxes(oracle, n, levels, order):
+    import qubatron_gb300 as qb
+    rng = np.random.default_rng(n + levels)
+    p = _points(n, levels, rng, order)
+    nodes = qb.build_octree(p, S, levels)
+    pos = rng.uniform(0.0, S, (3000, 3)).astype(np.float32)
+    d = (p[rng.integers(0, n, 3000)] - pos).astype(np.float32)
+    base = (0.0, S, S, S)
+    with qb.OctreeGLC(0) as up:
+        up.upload_octree(False, nodes)
+        want = up.trace_rays(pos, d, base, min(levels, 17))
+    for dynamic in (False, True):
+        with qb.OctreeGLC(0) as ctx:
+            for _ in range(2):  # the second build reuses what the first left
+                assert ctx.build_tree(dynamic, p, S, levels, first_index=0) == nodes.shape[0]
+            assert np.array_equal(ctx.download_tree(dynamic), nodes), dynamic
+            if not dynamic:
+                got = ctx.trace_rays(pos, d, base, min(levels, 17))
+                for k in ("status", "leaf", "visits"):
+                    assert np.array_equal(got[k], want[k]), k
