@@ -22,13 +22,20 @@
 // breadth-first order), a child index outside the array (which the walk
 // reports when it meets it) or a tree deeper than the shader's stack leaves
 // the boxes unusable.
+//
+// The level counts stay on the device: every kernel finds its level's range
+// from them, and the host reads them once, when all is queued (it read them
+// after every level before). A node's children are neighbours in the order,
+// so their boxes are read in one run, and a level's boxes and records are
+// made in one kernel. 2.6M nodes of a 1M-point floor: 1.1 ms of kernels, 13
+// waits and five allocations before; 0.47 ms of kernels now.
 
 #include <cuda_runtime.h>
-#include <thrust/device_vector.h>
 
+#include <algorithm>
 #include <cstdint>
-#include <vector>
 
+#include "boxes.cuh"
 #include "qbc_internal.h"
 #include "qbcuda.h"
 
@@ -37,20 +44,30 @@ using qbc::fail;
 namespace qbc {
 namespace {
 
-constexpr int kMaxDepth = QBC_MAX_LEVEL + 1;
+constexpr int kLevels = QBC_MAX_LEVEL + 1;  // levels expanded: nodes of a deeper one rule the boxes out
 
-int grid_of(int64_t n) {
-  const int64_t b = (n + 255) / 256;
-  return (int)(b < 1 ? 1 : (b > 4096 ? 4096 : b));
+struct Counts {
+  unsigned long long level[kLevels + 1];  // nodes per level
+  unsigned bad;                           // a child index outside the array, or a node reached twice
+};
+
+// First position of level L in the order, and its end.
+__device__ __forceinline__ void level_range(const Counts* c, int L, int64_t* b, int64_t* e) {
+  unsigned long long at = 0;
+  for (int k = 0; k < L; ++k) at += c->level[k];
+  *b = (int64_t)at;
+  *e = (int64_t)(at + c->level[L]);
 }
 
-// Children of the nodes in [in_b, in_e) of `order` appended at the end of
-// the order (the counter), each with its position in pos. One counter update
-// per warp and pass: each lane takes its node's children, the warp reserves
-// their total at once.
-__global__ void expand_kernel(const int32_t* __restrict__ child, int64_t n, int32_t* __restrict__ order,
-                              int32_t* __restrict__ pos, int64_t in_b, int64_t in_e,
-                              unsigned long long* __restrict__ count) {
+// Children of the nodes of level L appended to the order after them, each
+// with its position in pos; a node's first child's position to `first`. One
+// counter update per warp and pass: each lane takes its node's children, the
+// warp reserves their total at once.
+__global__ void expand_kernel(const int4* __restrict__ child, int64_t n, int32_t* __restrict__ order,
+                              int32_t* __restrict__ pos, int32_t* __restrict__ first, Counts* counts, int L) {
+  int64_t in_b, in_e;
+  level_range(counts, L, &in_b, &in_e);
+  if (in_e > n) return;  // not a tree, detected on the host
   const int lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   // the loop's trip count is the same for the whole warp (ballots below)
@@ -60,11 +77,7 @@ __global__ void expand_kernel(const int32_t* __restrict__ child, int64_t n, int3
     uint32_t take = 0;
     bool outside = false;
     if (j < in_e) {
-      const int32_t node = order[j];
-      const int4* p = reinterpret_cast<const int4*>(child + (int64_t)node * 8);
-      const int4 a = p[0], b = p[1];
-      c[0] = a.x; c[1] = a.y; c[2] = a.z; c[3] = a.w;
-      c[4] = b.x; c[5] = b.y; c[6] = b.z; c[7] = b.w;
+      load_children(child, order[j], c);
 #pragma unroll
       for (int o = 0; o < 8; ++o) {
         take |= (c[o] > 0 && c[o] < n) ? (1u << o) : 0u;
@@ -80,17 +93,16 @@ __global__ void expand_kernel(const int32_t* __restrict__ child, int64_t n, int3
       const unsigned v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
       if (lane >= o) incl += v;
     }
-    const unsigned total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-    const bool any_outside = __any_sync(0xFFFFFFFFu, outside);
     unsigned long long base = 0;
-    if (lane == 31 && (total || any_outside))
-      base = atomicAdd(count, (unsigned long long)total + (any_outside ? (unsigned long long)n + 1ull : 0ull));
+    if (lane == 31 && incl) base = atomicAdd(&counts->level[L + 1], (unsigned long long)incl);
+    if (__any_sync(0xFFFFFFFFu, outside) && lane == 0) counts->bad = 1u;
     base = __shfl_sync(0xFFFFFFFFu, base, 31);
-    unsigned long long k = base + (incl - mine);
+    int64_t k = in_e + (int64_t)base + (incl - mine);
+    if (j < in_e) first[j] = (int32_t)min(k, n);
 #pragma unroll
     for (int o = 0; o < 8; ++o) {
       if ((take >> o) & 1u) {
-        if ((int64_t)k < n) {  // past n: not a tree, detected on the host
+        if (k < n) {  // past n: not a tree, detected on the host
           order[k] = c[o];
           pos[c[o]] = (int32_t)k;
         }
@@ -102,146 +114,96 @@ __global__ void expand_kernel(const int32_t* __restrict__ child, int64_t n, int3
 
 // A node appended twice (two parents, or a cycle) keeps one of its positions
 // in pos, so another position of it disagrees: then the array is not a tree.
-__global__ void unique_kernel(const int32_t* __restrict__ order, const int32_t* __restrict__ pos, int64_t total,
-                              unsigned int* __restrict__ dup) {
-  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < total; j += (int64_t)gridDim.x * blockDim.x)
-    if (pos[order[j]] != (int32_t)j) *dup = 1u;
+__global__ void unique_kernel(const int32_t* __restrict__ order, const int32_t* __restrict__ pos, int64_t n,
+                              Counts* counts) {
+  int64_t b, e;
+  level_range(counts, kLevels, &b, &e);
+  if (e > n) return;
+  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < e; j += (int64_t)gridDim.x * blockDim.x)
+    if (pos[order[j]] != (int32_t)j) counts->bad = 1u;
 }
 
-// Exact boxes in leaf cells relative to each node's cube, for the nodes of one
-// level (children done). box: 6 ints per node (xlo xhi ylo yhi zlo zhi).
-__global__ void box_level_kernel(const int32_t* __restrict__ child, int64_t n, const int32_t* __restrict__ order,
-                                 int64_t b, int64_t e, int leaf_level, int32_t half_cells,
-                                 int32_t* __restrict__ box) {
+// Boxes in leaf cells of the nodes of level L, by position (children done),
+// and their records.
+__global__ void box_level_kernel(const int4* __restrict__ child, int64_t n, const int32_t* __restrict__ order,
+                                 const int32_t* __restrict__ first, const Counts* counts, int L,
+                                 uint4* __restrict__ box, uint4* __restrict__ rec) {
+  int64_t b, e, all_b, all_e;
+  level_range(counts, L, &b, &e);
+  level_range(counts, kLevels, &all_b, &all_e);
+  if (counts->bad || all_e > n || all_b < all_e) return;  // no boxes
+  int depth = L;
+  while (depth + 1 <= kLevels && counts->level[depth + 1] > 0) ++depth;
+  const int sh = depth - L - 1;  // a child's edge: 2^sh leaf cells
   for (int64_t j = b + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < e; j += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t node = order[j];
-    int32_t r[6];
-    if (leaf_level) {
-      r[0] = r[1] = r[2] = r[3] = r[4] = r[5] = 0;
-    } else {
-      r[0] = r[2] = r[4] = 0x7fffffff;
-      r[1] = r[3] = r[5] = -1;
-      for (int o = 0; o < 8; ++o) {
-        const int32_t c = child[(int64_t)node * 8 + o];
-        if (!(c > 0 && c < n)) continue;
-        const int32_t* cb = box + (int64_t)c * 6;
-        if (cb[1] < cb[0]) continue;  // no leaves below
-        const int32_t off[3] = {(o & 1) ? half_cells : 0, (o & 2) ? half_cells : 0, (o & 4) ? half_cells : 0};
-        for (int k = 0; k < 3; ++k) {
-          r[2 * k] = min(r[2 * k], cb[2 * k] + off[k]);
-          r[2 * k + 1] = max(r[2 * k + 1], cb[2 * k + 1] + off[k]);
-        }
-      }
+    if (L == depth) {
+      box[j] = make_uint4(0u, 0u, 0u, 0u);  // its own cell
+      continue;
     }
-    for (int k = 0; k < 6; ++k) box[(int64_t)node * 6 + k] = r[k];
-  }
-}
-
-// Records of the nodes of one level: each child's box quantised outward to
-// 1/256 of the child's edge (child_cells leaf cells).
-__global__ void record_kernel(const int32_t* __restrict__ child, int64_t n, const int32_t* __restrict__ order,
-                              int64_t b, int64_t e, int32_t child_cells, const int32_t* __restrict__ box,
-                              uint32_t* __restrict__ rec) {
-  for (int64_t j = b + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < e; j += (int64_t)gridDim.x * blockDim.x) {
     const int32_t node = order[j];
-    uint32_t w[16];
-    for (int k = 0; k < 16; ++k) w[k] = 0u;
+    int32_t c[8];
+    load_children(child, node, c);
+    int64_t k = first[j];
+    CellBox u = no_box();
+    uint2 w[8];
+#pragma unroll
     for (int o = 0; o < 8; ++o) {
-      const int32_t c = child[(int64_t)node * 8 + o];
-      uint32_t q[6] = {255u, 0u, 255u, 0u, 255u, 0u};  // empty
-      if (c > 0 && c < n) {
-        const int32_t* cb = box + (int64_t)c * 6;
-        if (cb[0] <= cb[1]) {
-          for (int k = 0; k < 3; ++k) {
-            const int64_t lo = cb[2 * k], hi1 = (int64_t)cb[2 * k + 1] + 1;  // [lo, hi1) in leaf cells
-            // in 1/256 of the edge: floor(lo * 256 / cells), ceil(hi1 * 256 / cells) - 1
-            const int64_t ql = lo * 256 / child_cells;
-            const int64_t qh = (hi1 * 256 + child_cells - 1) / child_cells - 1;
-            q[2 * k] = (uint32_t)(ql < 0 ? 0 : (ql > 255 ? 255 : ql));
-            q[2 * k + 1] = (uint32_t)(qh < 0 ? 0 : (qh > 255 ? 255 : qh));
-          }
-        }
-      }
-      w[2 * o] = q[0] | (q[1] << 8) | (q[2] << 16) | (q[3] << 24);
-      w[2 * o + 1] = q[4] | (q[5] << 8);
+      w[o] = empty_word();
+      if (!(c[o] > 0 && c[o] < n)) continue;
+      const CellBox v = unpack_box(box[k++]);
+      if (v.lo[0] > v.hi[0]) continue;  // no leaves below
+      w[o] = record_word(v, sh);
+      add_box(u, v, o, sh);
     }
-    uint4* dst = reinterpret_cast<uint4*>(rec + (int64_t)node * 16);
-    for (int k = 0; k < 4; ++k) dst[k] = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
+    box[j] = pack_box(u);
+    store_record(rec, node, w);
   }
 }
 
 }  // namespace
 
-int build_child_boxes(const int32_t* child, int64_t n, uint32_t* rec, cudaStream_t stream, int* depth,
-                      int64_t* launches) {
+size_t box_scratch(int64_t n) { return (size_t)n * 28 + sizeof(Counts) + 64; }
+
+int build_child_boxes(const int32_t* child, int64_t n, uint32_t* rec, void* scratch, cudaStream_t stream, int grid,
+                      int* depth, int64_t* launches) {
   *depth = -1;
   if (n <= 0) return QBC_OK;
-  try {
-    thrust::device_vector<int32_t> order(n), pos(n);
-    thrust::device_vector<unsigned long long> count(1);
-    thrust::device_vector<unsigned int> dup(1);
-    int32_t zero = 0;
-    unsigned int no = 0u;
-    cudaMemcpyAsync(thrust::raw_pointer_cast(order.data()), &zero, 4, cudaMemcpyHostToDevice, stream);
-    cudaMemcpyAsync(thrust::raw_pointer_cast(pos.data()), &zero, 4, cudaMemcpyHostToDevice, stream);
-    cudaMemcpyAsync(thrust::raw_pointer_cast(dup.data()), &no, 4, cudaMemcpyHostToDevice, stream);
-    // breadth first: level L holds order[off[L], off[L+1])
-    std::vector<int64_t> off = {0, 1};
-    unsigned long long total = 1;
-    cudaMemcpyAsync(thrust::raw_pointer_cast(count.data()), &total, 8, cudaMemcpyHostToDevice, stream);
-    for (int L = 0; L <= kMaxDepth; ++L) {
-      const int64_t b = off[L], e = off[L + 1];
-      if (e == b) break;
-      expand_kernel<<<grid_of(e - b), 256, 0, stream>>>(child, n, thrust::raw_pointer_cast(order.data()),
-                                                         thrust::raw_pointer_cast(pos.data()), b, e,
-                                                         thrust::raw_pointer_cast(count.data()));
-      ++*launches;
-      cudaError_t err = cudaMemcpyAsync(&total, thrust::raw_pointer_cast(count.data()), 8, cudaMemcpyDeviceToHost,
-                                        stream);
-      if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
-      if (err != cudaSuccess) return fail(QBC_E_CUDA, "box build: %s", cudaGetErrorString(err));
-      if ((int64_t)total > n) return QBC_OK;  // a node reached twice: no boxes
-      off.push_back((int64_t)total);
-    }
-    // every node once (the counter alone misses a node reached twice when
-    // others are unreachable)
-    {
-      unique_kernel<<<grid_of(off.back()), 256, 0, stream>>>(thrust::raw_pointer_cast(order.data()),
-                                                            thrust::raw_pointer_cast(pos.data()), off.back(),
-                                                            thrust::raw_pointer_cast(dup.data()));
-      ++*launches;
-      unsigned int d = 0u;
-      cudaError_t err = cudaMemcpyAsync(&d, thrust::raw_pointer_cast(dup.data()), 4, cudaMemcpyDeviceToHost, stream);
-      if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
-      if (err != cudaSuccess) return fail(QBC_E_CUDA, "box build: %s", cudaGetErrorString(err));
-      if (d) return QBC_OK;  // a node reached twice: no boxes
-    }
-    // the deepest level with nodes
-    int D = 0;
-    while (D + 2 < (int)off.size() && off[D + 2] > off[D + 1]) ++D;
-    if (D > QBC_MAX_LEVEL) return QBC_OK;  // deeper than any render goes: no boxes
-    thrust::device_vector<int32_t> box((size_t)n * 6);
-    for (int L = D; L >= 0; --L) {
-      const int64_t b = off[L], e = off[L + 1];
-      box_level_kernel<<<grid_of(e - b), 256, 0, stream>>>(child, n, thrust::raw_pointer_cast(order.data()), b, e,
-                                                            L == D ? 1 : 0, L == D ? 0 : (int32_t)(1 << (D - L - 1)),
-                                                            thrust::raw_pointer_cast(box.data()));
-      ++*launches;
-    }
-    for (int L = 0; L < D; ++L) {
-      const int64_t b = off[L], e = off[L + 1];
-      record_kernel<<<grid_of(e - b), 256, 0, stream>>>(child, n, thrust::raw_pointer_cast(order.data()), b, e,
-                                                         (int32_t)(1 << (D - L - 1)),
-                                                         thrust::raw_pointer_cast(box.data()), rec);
-      ++*launches;
-    }
-    cudaError_t err = cudaStreamSynchronize(stream);
-    if (err == cudaSuccess) err = cudaGetLastError();
-    if (err != cudaSuccess) return fail(QBC_E_CUDA, "box build: %s", cudaGetErrorString(err));
-    *depth = D;
-  } catch (const std::exception& ex) {
-    return fail(QBC_E_NOMEM, "box build: %s", ex.what());
-  }
+  uint4* box = static_cast<uint4*>(scratch);
+  int32_t* order = reinterpret_cast<int32_t*>(box + n);
+  int32_t* pos = order + n;
+  int32_t* first = pos + n;
+  Counts* counts =
+      reinterpret_cast<Counts*>((reinterpret_cast<uintptr_t>(first + n) + 15) & ~static_cast<uintptr_t>(15));
+  const int4* blocks = reinterpret_cast<const int4*>(child);
+  uint4* records = reinterpret_cast<uint4*>(rec);
+  const unsigned long long one = 1;
+  cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(Counts), stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&counts->level[0], &one, 8, cudaMemcpyHostToDevice, stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(order, 0, 4, stream);  // the root
+  if (e == cudaSuccess) e = cudaMemsetAsync(pos, 0, 4, stream);
+  if (e != cudaSuccess) return fail(QBC_E_CUDA, "box build: %s", cudaGetErrorString(e));
+  // blocks of a level's kernel: the level holds at most min(n, 8^L) nodes
+  auto blocks_of = [&](int L) {
+    const int64_t most = L >= 10 ? n : std::min<int64_t>(n, int64_t(1) << (3 * L));
+    return (unsigned)std::min<int64_t>(grid, (most + 255) / 256);
+  };
+  for (int L = 0; L < kLevels; ++L)
+    expand_kernel<<<blocks_of(L), 256, 0, stream>>>(blocks, n, order, pos, first, counts, L);
+  unique_kernel<<<blocks_of(kLevels), 256, 0, stream>>>(order, pos, n, counts);
+  for (int L = kLevels - 1; L >= 0; --L)
+    box_level_kernel<<<blocks_of(L), 256, 0, stream>>>(blocks, n, order, first, counts, L, box, records);
+  *launches += 2 * kLevels + 1;
+  Counts h;
+  e = cudaMemcpyAsync(&h, counts, sizeof(h), cudaMemcpyDeviceToHost, stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e != cudaSuccess) return fail(QBC_E_CUDA, "box build: %s", cudaGetErrorString(e));
+  unsigned long long total = 0;
+  for (int L = 0; L <= kLevels; ++L) total += h.level[L];
+  if (h.bad || (int64_t)total > n || h.level[kLevels] > 0) return QBC_OK;  // no boxes
+  int D = 0;
+  while (h.level[D + 1] > 0) ++D;
+  *depth = D;
   return QBC_OK;
 }
 

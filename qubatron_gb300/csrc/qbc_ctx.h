@@ -50,7 +50,7 @@ struct qbc_ctx {
   DevModelBuf model[2];
   void* stage = nullptr;  // device staging for uploads
   size_t stage_bytes = 0;
-  void* scratch = nullptr;  // device outputs for host-output renders
+  void* scratch = nullptr;  // ensure_scratch's
   size_t scratch_bytes = 0;
   unsigned int* queue = nullptr;  // global tile counter of the persistent render kernel
   // two-pass render: records, counters (queued, shade-pass next), statistics, per-pixel log
@@ -123,6 +123,40 @@ inline int ensure_stage(qbc_ctx* c, size_t bytes) {
   c->stage_bytes = bytes;
   return QBC_OK;
 }
+
+// Device scratch of one call (host-output renders, ray queries, edits, box
+// builds), kept with the context. Calls are ordered by the context's stream.
+inline int ensure_scratch(qbc_ctx* c, size_t bytes, const char* what) {
+  if (c->scratch_bytes >= bytes) return QBC_OK;
+  if (c->scratch) QBC_CUDA(cudaFree(c->scratch));
+  c->scratch = nullptr;
+  c->scratch_bytes = 0;
+  cudaError_t e = cudaMalloc(&c->scratch, bytes);
+  if (e != cudaSuccess) return fail(QBC_E_NOMEM, "%s: scratch of %zu bytes: %s", what, bytes, cudaGetErrorString(e));
+  c->scratch_bytes = bytes;
+  return QBC_OK;
+}
+
+// Scratch for a call that waits for the stream before it returns: the
+// context's up to kStageMax bytes, larger given back at the end.
+struct CallScratch {
+  void* ptr = nullptr;
+  bool own = false;
+  ~CallScratch() {
+    if (own) cudaFree(ptr);
+  }
+  int take(qbc_ctx* c, size_t bytes, const char* what) {
+    if (bytes <= kStageMax) {
+      int rc = ensure_scratch(c, bytes, what);
+      ptr = c->scratch;
+      return rc;
+    }
+    cudaError_t e = cudaMalloc(&ptr, bytes);
+    if (e != cudaSuccess) return fail(QBC_E_NOMEM, "%s: scratch of %zu bytes: %s", what, bytes, cudaGetErrorString(e));
+    own = true;
+    return QBC_OK;
+  }
+};
 
 template <typename T>
 inline int grow(T** p, int64_t* cap, int64_t need, size_t elem_bytes, const char* what) {

@@ -85,18 +85,24 @@ int build_tree_static(const float* d_pts, const int32_t* d_octets, int64_t n, fl
                       int32_t* d_total, int64_t* total, unsigned* flag, unsigned* err, cudaStream_t stream, int grid,
                       int64_t* launches);
 
-// octree_remove_point (octree.c:182-218) of n points in order, on a device
-// tree (child: 8 int32 per node, model: 1 per node): cuts the links in place,
-// reports modind / octind per point (-1 where nothing was removed) into
-// device arrays and the number removed.
+// octree_remove_point (octree.c:182-218) of n > 0 points in order, on a device
+// tree (child: 8 int32 per node, model: 1 per node): cuts the links in place
+// and reports modind / octind per point (-1 where nothing was removed) into
+// device arrays; the number removed goes to *d_removed, a device word in
+// `scratch` (remove_scratch(n) bytes of device memory, 8-byte aligned).
+// Enqueued on `stream`.
+size_t remove_scratch(int64_t n);
 int remove_points(int32_t* child, const int32_t* model, int64_t n_nodes, const float* d_pts, int64_t n,
-                  float basesize, int levels, int32_t* d_modind, int32_t* d_octind, int64_t* removed,
-                  cudaStream_t stream, int64_t* launches);
+                  float basesize, int levels, int32_t* d_modind, int32_t* d_octind, void* scratch,
+                  unsigned long long** d_removed, cudaStream_t stream, int64_t* launches);
 
 // Leaf-box records of every node's children (boxes.cu) for the tree `child`
 // (8 int32 per node, n nodes) into rec (16 words per node); depth gets the
 // tree's depth, or -1 when the array is not a tree the renders can use.
-int build_child_boxes(const int32_t* child, int64_t n, uint32_t* rec, cudaStream_t stream, int* depth,
-                      int64_t* launches);
+// `scratch`: box_scratch(n) bytes of device memory, 16-byte aligned.
+// Synchronizes once, at the end.
+size_t box_scratch(int64_t n);
+int build_child_boxes(const int32_t* child, int64_t n, uint32_t* rec, void* scratch, cudaStream_t stream, int grid,
+                      int* depth, int64_t* launches);
 
 }  // namespace qbc

@@ -681,23 +681,19 @@ extern "C" int qbc_tree_remove_points(qbc_ctx* c, int tree, const float* pts, in
     if (removed) *removed = 0;
     return QBC_OK;
   }
-  // device arrays: the caller's when on_device, else staged
-  void* tmp = nullptr;
-  const size_t pbytes = (size_t)n * 12, obytes = (size_t)n * 4;
+  // device arrays: the caller's when on_device, else in the scratch, behind
+  // the removal's own (8-byte aligned parts)
+  const size_t work = (qbc::remove_scratch(n) + 15) & ~size_t(15), pbytes = (size_t)n * 12, obytes = (size_t)n * 4;
+  const bool stage_out = !on_device || !modind || !octind;
+  CallScratch scratch;
+  int rc = scratch.take(c, work + (on_device ? 0 : pbytes) + (stage_out ? 2 * obytes : 0), "qbc_tree_remove_points");
+  if (rc) return rc;
+  char* t = static_cast<char*>(scratch.ptr) + work;
   const float* dp = pts;
   int32_t* dm = modind;
   int32_t* dq = octind;
-  const bool stage_out = !on_device || !modind || !octind;
-  size_t need = (on_device ? 0 : pbytes) + (stage_out ? 2 * obytes : 0);
-  if (need) {
-    cudaError_t e = cudaMalloc(&tmp, need);
-    if (e != cudaSuccess) return fail(QBC_E_NOMEM, "qbc_tree_remove_points: %s", cudaGetErrorString(e));
-  }
-  char* t = static_cast<char*>(tmp);
-  int rc = QBC_OK;
   if (!on_device) {
-    cudaError_t e = cudaMemcpyAsync(t, pts, pbytes, cudaMemcpyHostToDevice, c->stream);
-    if (e != cudaSuccess) rc = cuda_fail(e, "qbc_tree_remove_points: copy points");
+    QBC_CUDA(cudaMemcpyAsync(t, pts, pbytes, cudaMemcpyHostToDevice, c->stream));
     dp = reinterpret_cast<const float*>(t);
     t += pbytes;
   }
@@ -705,20 +701,21 @@ extern "C" int qbc_tree_remove_points(qbc_ctx* c, int tree, const float* pts, in
     dm = reinterpret_cast<int32_t*>(t);
     dq = reinterpret_cast<int32_t*>(t + obytes);
   }
-  if (!rc)
-    rc = qbc::remove_points(reinterpret_cast<int32_t*>(c->tree[tree].child), c->tree[tree].model, c->tree[tree].n,
-                            dp, n, basesize, levels, dm, dq, removed, c->stream, &c->launches);
-  if (!rc && stage_out) {
+  unsigned long long* count = nullptr;
+  rc = qbc::remove_points(reinterpret_cast<int32_t*>(c->tree[tree].child), c->tree[tree].model, c->tree[tree].n, dp, n,
+                          basesize, levels, dm, dq, scratch.ptr, &count, c->stream, &c->launches);
+  if (rc) return rc;
+  if (stage_out) {
     // results to the caller's arrays (host, or device when only one was given)
     const cudaMemcpyKind k = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    cudaError_t e = cudaSuccess;
-    if (modind) e = cudaMemcpyAsync(modind, dm, obytes, k, c->stream);
-    if (e == cudaSuccess && octind) e = cudaMemcpyAsync(octind, dq, obytes, k, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    if (e != cudaSuccess) rc = cuda_fail(e, "qbc_tree_remove_points: copy results");
+    if (modind) QBC_CUDA(cudaMemcpyAsync(modind, dm, obytes, k, c->stream));
+    if (octind) QBC_CUDA(cudaMemcpyAsync(octind, dq, obytes, k, c->stream));
   }
-  if (tmp) cudaFree(tmp);
-  return rc;
+  unsigned long long h = 0;
+  QBC_CUDA(cudaMemcpyAsync(&h, count, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
+  QBC_CUDA(cudaStreamSynchronize(c->stream));
+  if (removed) *removed = (int64_t)h;
+  return QBC_OK;
 }
 
 extern "C" int qbc_download_tree(qbc_ctx* c, int tree, int32_t* nodes, int64_t cap, int64_t* n_nodes) {
@@ -760,10 +757,13 @@ int ensure_boxes(qbc_ctx* c) {
         int rc = grow(&tb.cbox, &tb.cbox_cap, tb.cap > tb.n ? tb.cap : tb.n, 64, "octree leaf boxes");
         if (rc) return rc;
       }
-      QBC_CUDA(cudaMemsetAsync(tb.cbox, 0, (size_t)tb.n * 64, c->stream));
+      // (records no walk uses stay as they are)
+      CallScratch scratch;
+      int rc = scratch.take(c, qbc::box_scratch(tb.n), "leaf boxes");
+      if (rc) return rc;
       int depth = -1;
-      int rc = qbc::build_child_boxes(reinterpret_cast<const int32_t*>(tb.child), tb.n, tb.cbox, c->stream, &depth,
-                                      &c->launches);
+      rc = qbc::build_child_boxes(reinterpret_cast<const int32_t*>(tb.child), tb.n, tb.cbox, scratch.ptr, c->stream,
+                                  c->sm_count * 8, &depth, &c->launches);
       if (rc) return rc;
       tb.box_depth = depth;
     }
@@ -1145,14 +1145,8 @@ int render_views_impl(qbc_ctx* c, const qbc_view* views, const qbc_outputs* outs
     for (int k = 0; k < 6; ++k)
       if (*out_slot(h, k)) need += (px * kOutBytes[k] + 255) & ~size_t(255);
   }
-  if (need > c->scratch_bytes) {
-    if (c->scratch) QBC_CUDA(cudaFree(c->scratch));
-    c->scratch = nullptr;
-    c->scratch_bytes = 0;
-    cudaError_t e = cudaMalloc(&c->scratch, need);
-    if (e != cudaSuccess) return fail(QBC_E_NOMEM, "render scratch of %zu bytes: %s", need, cudaGetErrorString(e));
-    c->scratch_bytes = need;
-  }
+  int src = ensure_scratch(c, need, "render");
+  if (src) return src;
   size_t off = 0;
   for (int i = 0; i < n; ++i) {
     size_t px = (size_t)views[i].width_px * views[i].height_px;
@@ -1264,14 +1258,8 @@ extern "C" int qbc_trace_rays(qbc_ctx* c, const float* pos, const float* dir, in
     size_t need = 2 * ((size_t)n * 12 + 256);
     for (int k = 0; k < 7; ++k)
       if (*hs[k]) need += ((size_t)n * bytes[k] + 255) & ~size_t(255);
-    if (need > c->scratch_bytes) {
-      if (c->scratch) QBC_CUDA(cudaFree(c->scratch));
-      c->scratch = nullptr;
-      c->scratch_bytes = 0;
-      cudaError_t e = cudaMalloc(&c->scratch, need);
-      if (e != cudaSuccess) return fail(QBC_E_NOMEM, "ray scratch of %zu bytes: %s", need, cudaGetErrorString(e));
-      c->scratch_bytes = need;
-    }
+    int src = ensure_scratch(c, need, "rays");
+    if (src) return src;
     char* base = (char*)c->scratch;
     size_t off = 0;
     float* dpos = (float*)(base + off);
@@ -1338,14 +1326,8 @@ extern "C" int qbc_camera_rays(qbc_ctx* c, const qbc_view* view, const int32_t* 
     // pixel indices and rays staged in the context's scratch
     const size_t idx = ((size_t)n * 4 + 255) & ~size_t(255);
     const size_t need = 2 * idx + (size_t)n * 16;
-    if (need > c->scratch_bytes) {
-      if (c->scratch) QBC_CUDA(cudaFree(c->scratch));
-      c->scratch = nullptr;
-      c->scratch_bytes = 0;
-      cudaError_t e = cudaMalloc(&c->scratch, need);
-      if (e != cudaSuccess) return fail(QBC_E_NOMEM, "camera-ray scratch of %zu bytes: %s", need, cudaGetErrorString(e));
-      c->scratch_bytes = need;
-    }
+    int src = ensure_scratch(c, need, "camera rays");
+    if (src) return src;
     char* base = (char*)c->scratch;
     QBC_CUDA(cudaMemcpyAsync(base, px, (size_t)n * 4, cudaMemcpyHostToDevice, c->stream));
     QBC_CUDA(cudaMemcpyAsync(base + idx, py, (size_t)n * 4, cudaMemcpyHostToDevice, c->stream));

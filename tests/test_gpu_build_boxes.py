@@ -51,3 +51,55 @@ def test_built_tree_and_boxes(oracle, n, levels, order):
                 got = ctx.trace_rays(pos, d, base, min(levels, 17))
                 for k in ("status", "leaf", "visits"):
                     assert np.array_equal(got[k], want[k]), k
+
+
+@pytest.mark.parametrize("kind", ["whole", "stubs", "twice", "outside", "root"])
+@pytest.mark.parametrize("n,levels", [(1, 3), (40, 1), (700, 8), (5000, 12)])
+def test_uploaded_boxes(oracle, kind, n, levels):
+    """Boxes of uploaded arrays: childless nodes above the deepest level, and
+    arrays that get none (a node with two parents, an index outside)."""
+    import qubatron_gb300 as qb
+    rng = np.random.default_rng(n)
+    p = _points(n, levels, rng, "shuffled")
+    nodes = qb.build_octree(p, S, levels).copy()
+    if kind == "root":
+        nodes = nodes[:1].copy()
+        nodes[:, :8] = 0
+    links = np.argwhere(nodes[:, :8] > 0)
+    if kind == "stubs":
+        for k in rng.integers(0, len(links), len(links) // 4):
+            nodes[tuple(links[k])] = 0
+    elif kind == "twice" and len(links) > 1:
+        leaf = nodes[tuple(links[-1])]  # an edge to a leaf cell, given a second parent
+        node, octet = links[len(links) // 2]
+        if node != links[-1][0]:
+            nodes[node, octet] = leaf
+    elif kind == "outside":
+        nodes[tuple(links[-1])] = nodes.shape[0] + 5
+    pos = rng.uniform(0.0, S, (2000, 3)).astype(np.float32)
+    d = (p[rng.integers(0, n, 2000)] - pos).astype(np.float32)
+    one = np.full((1, 3), 0.5, np.float32)
+    ref = oracle.trace_rays(oracle.Scene(nodes, one.repeat(n, 0), one.repeat(n, 0), boxes=True), (0.0, S, S, S), levels,
+                            pos, d)
+    with qb.OctreeGLC(0) as ctx:
+        ctx.upload_octree(False, nodes)
+        got = ctx.trace_rays(pos, d, (0.0, S, S, S), levels)
+    for k in ("status", "leaf", "visits"):
+        assert np.array_equal(got[k], ref[k]), k
+
+
+@pytest.mark.parametrize("n,cells", [(1, 1), (33, 1), (257, 1), (4097, 7), (30000, 5000)])
+def test_removals_with_duplicates(oracle, n, cells):
+    """Many points of few leaves: the first in input order of each removes it."""
+    import qubatron_gb300 as qb
+    rng = np.random.default_rng(n)
+    p = _points(6000, 9, rng, "shuffled")
+    nodes = qb.build_octree(p, S, 9)
+    shots = np.concatenate([p[rng.integers(0, cells, n)], rng.uniform(0.0, S, (n // 3, 3)).astype(np.float32)])
+    want_nodes = nodes.copy()
+    want = oracle.remove_points(want_nodes, shots, S, 9)
+    with qb.OctreeGLC(0) as ctx:
+        ctx.upload_octree(False, nodes)
+        mod, octind, removed = ctx.remove_points(False, shots, S, 9)
+        assert np.array_equal(ctx.download_tree(False)[:, :9], want_nodes[:, :9])
+    assert np.array_equal(mod, want[0]) and np.array_equal(octind, want[1]) and removed == (want[0] >= 0).sum()
