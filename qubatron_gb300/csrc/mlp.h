@@ -18,7 +18,6 @@ constexpr int kGate = 3;      // output 3: logit of "the shadow ray is occluded 
 constexpr int kOutUsed = 4;
 constexpr int kOutPad = 16;
 constexpr float kGateWeight = 0.05f;  // weight of the gate's cross-entropy in the loss
-constexpr int64_t kChunkRows = 1 << 20;  // inference rows per pass through the work buffer
 
 int64_t param_offset(int layer, bool bias);  // floats into the master array
 int64_t param_count();
@@ -30,8 +29,8 @@ struct Net {
   float* grad = nullptr;
   float* m = nullptr;            // Adam moments
   float* v = nullptr;
-  void* work = nullptr;          // activations of a batch
-  int64_t work_rows = 0;
+  float* partial = nullptr;      // weight gradients of each block of a gradient
+  int sms = 0;
   int64_t step_count = 0;
   bool ready = false;
   unsigned* err = nullptr;       // device error word of the owning context
@@ -40,13 +39,16 @@ struct Net {
   int set(const float* host, cudaStream_t s);
   int get(float* host, cudaStream_t s) const;
   int sync_weights(cudaStream_t s);
-  int ensure_work(int64_t rows);
-  // out: rows x kOutPad fp32; keep: retain activations for gradient()
-  int forward(const __nv_bfloat16* X, int64_t rows, float* out, cudaStream_t s, bool keep = false);
-  // loss (device float, mean over rows) and parameter gradient into grad
-  int gradient(const __nv_bfloat16* X, const float* tlab, const int8_t* kind, int64_t rows, float* loss,
-               cudaStream_t s);
-  int adam(float lr, cudaStream_t s);
+  // loss (device float, mean over rows of 45 floats) and its parameter
+  // gradient into grad
+  int gradient(const float* X, const float* tlab, const int8_t* kind, int64_t rows, float* loss, cudaStream_t s);
+  // one step of Adam on `rows` seeded picks of a training set of `samples`
+  // bf16 rows of kIn; the step's loss to *loss (device)
+  int train_step(const __nv_bfloat16* X, const float* tlab, const int8_t* kind, int64_t samples, uint64_t seed,
+                 int64_t rows, float lr, float* loss, cudaStream_t s);
+  // gradients of `rows` rows of src, by block, into partial
+  template <class Src>
+  int partials(const Src& src, int64_t rows, int* blocks, cudaStream_t s);
   void release();
 };
 

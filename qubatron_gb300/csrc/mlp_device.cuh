@@ -23,6 +23,16 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// Features 8 c .. 8 c + 7 of row r of a matrix of kInUsed floats a row, as the
+// network's bf16 inputs (zero past the last).
+__device__ __forceinline__ uint4 float_features(const float* x, uint32_t r, int c) {
+  const float* p = x + (size_t)r * kInUsed + 8 * c;
+  float f[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) f[k] = 8 * c + k < kInUsed ? p[k] : 0.0f;
+  return make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+}
+
 constexpr int kLdIn = kIn + 8;  // padded feature rows a Src loads (bytes a multiple of 16)
 
 // ---- fused inference on the 5th-generation tensor cores (tcgen05) ----

@@ -119,10 +119,10 @@ struct RecordRows {
   }
 };
 
-// Fused-network rows over a bf16 feature matrix (kIn per row) -> kOutUsed
-// floats per row.
+// Fused-network rows over a matrix of 45 floats a row -> kOutUsed floats per
+// row.
 struct MatrixRows {
-  const bf16* X;
+  const float* X;
   float* out;
   uint32_t m;
   __device__ __forceinline__ uint32_t rows() const { return m; }
@@ -131,39 +131,15 @@ struct MatrixRows {
     for (int e = lane; e < 16 * kVec; e += 32) {
       const int r = e / kVec, c = e % kVec;
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if ((uint32_t)r < n) v = reinterpret_cast<const uint4*>(X + (size_t)(r0 + r) * qbc::mlp::kIn)[c];
+      if ((uint32_t)r < n) v = qbc::mlp::float_features(X, r0 + r, c);
       *reinterpret_cast<uint4*>(x + r * qbc::mlp::kLdIn + c * 8) = v;
     }
   }
   __device__ __forceinline__ void store(uint32_t r, const float* o) const {
-    for (int k = 0; k < qbc::mlp::kOutUsed; ++k) out[(size_t)r * qbc::mlp::kOutUsed + k] = o[k];
+    reinterpret_cast<float4*>(out)[r] = make_float4(o[0], o[1], o[2], o[3]);
   }
 };
-
-// Random minibatch of the training set.
-__global__ void gather_kernel(const bf16* __restrict__ X, const float* __restrict__ tl,
-                              const int8_t* __restrict__ kind, int64_t n, int64_t rows, uint64_t seed,
-                              bf16* __restrict__ bx, float* __restrict__ bt, int8_t* __restrict__ bk) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < rows; i += (int64_t)gridDim.x * blockDim.x) {
-    uint64_t z = seed + 0x9E3779B97F4A7C15ull * (uint64_t)(i + 1);
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-    z ^= z >> 31;
-    const int64_t j = (int64_t)(z % (uint64_t)n);
-    for (int k = 0; k < qbc::mlp::kIn; ++k) bx[i * qbc::mlp::kIn + k] = X[j * qbc::mlp::kIn + k];
-    bt[i] = tl[j];
-    bk[i] = kind[j];
-  }
-}
-
-bf16 host_bf16(float f) {
-  // round to nearest even (NaN kept quiet)
-  uint32_t u;
-  std::memcpy(&u, &f, 4);
-  if ((u & 0x7fffffffu) > 0x7f800000u) return __ushort_as_bfloat16((unsigned short)((u >> 16) | 0x40));
-  u += 0x7fffu + ((u >> 16) & 1u);
-  return __ushort_as_bfloat16((unsigned short)(u >> 16));
-}
+static_assert(qbc::mlp::kOutUsed == 4, "one float4 a row");
 
 // One launch of the network over `src`'s rows on the tcgen05 tensor cores: a
 // persistent grid of one block per SM, each staging the weights once.
@@ -250,20 +226,6 @@ int propose_mlp(qbc_ctx* c, const qbc::Batch& b, const qbc::Wave& w) {
 // Occluder-proposal network: C ABI
 // ---------------------------------------------------------------------------
 
-namespace {
-// Host rows of 45 floats -> device bf16 rows of 48.
-int upload_features(qbc_ctx* c, const float* x, int64_t m, bf16** out) {
-  std::vector<bf16> h((size_t)m * qbc::mlp::kIn);
-  for (int64_t i = 0; i < m; ++i)
-    for (int k = 0; k < qbc::mlp::kIn; ++k)
-      h[(size_t)i * qbc::mlp::kIn + k] = host_bf16(k < qbc::mlp::kInUsed ? x[i * qbc::mlp::kInUsed + k] : 0.0f);
-  cudaError_t e = cudaMalloc(out, h.size() * 2);
-  if (e != cudaSuccess) return fail(QBC_E_NOMEM, "proposal features: %s", cudaGetErrorString(e));
-  QBC_CUDA(cudaMemcpyAsync(*out, h.data(), h.size() * 2, cudaMemcpyHostToDevice, c->stream));
-  return QBC_OK;
-}
-}  // namespace
-
 static_assert(QBC_PROPOSAL_PARAMS == 41360, "parameter count");
 
 extern "C" int qbc_proposal_collect(qbc_ctx* c, const qbc_view* views, int n, int64_t* samples) {
@@ -336,28 +298,18 @@ extern "C" int qbc_proposal_train(qbc_ctx* c, const qbc_train_opts* opts, qbc_tr
     int rc = c->net.init(opts->seed, c->stream);
     if (rc) return rc;
   }
-  const int64_t B = opts->batch;
-  bf16* bx = nullptr;
-  float* bt = nullptr;
-  int8_t* bk = nullptr;
   float* dloss = nullptr;
-  cudaError_t e = cudaMalloc(&bx, (size_t)B * qbc::mlp::kIn * 2);
-  if (e == cudaSuccess) e = cudaMalloc(&bt, (size_t)B * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&bk, (size_t)B);
-  if (e == cudaSuccess) e = cudaMalloc(&dloss, 4);
+  cudaError_t e = cudaMalloc(&dloss, 4);
   int rc = QBC_OK;
   if (e != cudaSuccess) rc = fail(QBC_E_NOMEM, "qbc_proposal_train: %s", cudaGetErrorString(e));
   float first = 0.0f, last = 0.0f;
   int nlast = 0;
   for (int step = 0; step < opts->steps && rc == QBC_OK; ++step) {
-    gather_kernel<<<launch_grid(c, B), 256, 0, c->stream>>>(c->ds_x, c->ds_t, c->ds_kind, n, B,
-                                                            opts->seed * 1000003ull + (uint64_t)step, bx, bt, bk);
     const int64_t l0 = qbc::mlp::launches();
-    rc = c->net.gradient(bx, bt, bk, B, dloss, c->stream);
+    rc = c->net.train_step(c->ds_x, c->ds_t, c->ds_kind, n, opts->seed * 1000003ull + (uint64_t)step, opts->batch,
+                           opts->lr, dloss, c->stream);
     if (rc) break;
-    rc = c->net.adam(opts->lr, c->stream);
-    if (rc) break;
-    c->launches += 1 + (qbc::mlp::launches() - l0);
+    c->launches += qbc::mlp::launches() - l0;
     if (step == 0 || step >= opts->steps - 10) {
       float l = 0.0f;
       e = cudaMemcpyAsync(&l, dloss, 4, cudaMemcpyDeviceToHost, c->stream);
@@ -374,9 +326,6 @@ extern "C" int qbc_proposal_train(qbc_ctx* c, const qbc_train_opts* opts, qbc_tr
     }
   }
   cudaStreamSynchronize(c->stream);
-  cudaFree(bx);
-  cudaFree(bt);
-  cudaFree(bk);
   cudaFree(dloss);
   if (rc) return rc;
   if (stats) {
@@ -426,25 +375,19 @@ extern "C" int qbc_proposal_eval(qbc_ctx* c, const float* x, int64_t m, float* o
   if (!c->net.ready) return fail(QBC_E_STATE, "qbc_proposal_eval: no network");
   if (m == 0) return QBC_OK;
   QBC_CUDA(cudaSetDevice(c->device));
-  bf16* dx = nullptr;
-  int rc = upload_features(c, x, m, &dx);
+  const size_t in = ((size_t)m * qbc::mlp::kInUsed * 4 + 255) & ~size_t(255), outb = (size_t)m * qbc::mlp::kOutUsed * 4;
+  CallScratch scratch;
+  int rc = scratch.take(c, in + outb, "qbc_proposal_eval");
   if (rc) return rc;
-  float* dout = nullptr;
-  cudaError_t e = cudaMalloc(&dout, (size_t)m * qbc::mlp::kOutUsed * 4);
-  if (e != cudaSuccess) {
-    cudaFree(dx);
-    return fail(QBC_E_NOMEM, "qbc_proposal_eval: %s", cudaGetErrorString(e));
-  }
+  float* dx = static_cast<float*>(scratch.ptr);
+  float* dout = reinterpret_cast<float*>(static_cast<char*>(scratch.ptr) + in);
+  QBC_CUDA(cudaMemcpyAsync(dx, x, (size_t)m * qbc::mlp::kInUsed * 4, cudaMemcpyHostToDevice, c->stream));
   MatrixRows src{dx, dout, (uint32_t)m};
   rc = launch_fused(c, src, 1);
-  if (!rc) {
-    e = cudaMemcpyAsync(out, dout, (size_t)m * qbc::mlp::kOutUsed * 4, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    if (e != cudaSuccess) rc = fail(QBC_E_CUDA, "qbc_proposal_eval: %s", cudaGetErrorString(e));
-  }
-  cudaFree(dx);
-  cudaFree(dout);
-  return rc;
+  if (rc) return rc;
+  QBC_CUDA(cudaMemcpyAsync(out, dout, outb, cudaMemcpyDeviceToHost, c->stream));
+  QBC_CUDA(cudaStreamSynchronize(c->stream));
+  return QBC_OK;
 }
 
 extern "C" int qbc_proposal_gradient(qbc_ctx* c, const float* x, const float* t, const int8_t* kind, int64_t m,
@@ -453,29 +396,28 @@ extern "C" int qbc_proposal_gradient(qbc_ctx* c, const float* x, const float* t,
   if (!c || m <= 0 || !x || !t || !kind || !loss || !grad) return fail(QBC_E_ARG, "qbc_proposal_gradient: bad argument");
   if (!c->net.ready) return fail(QBC_E_STATE, "qbc_proposal_gradient: no network");
   QBC_CUDA(cudaSetDevice(c->device));
-  bf16* dx = nullptr;
-  int rc = upload_features(c, x, m, &dx);
+  auto align = [](size_t b) { return (b + 255) & ~size_t(255); };
+  const size_t xb = (size_t)m * qbc::mlp::kInUsed * 4, tb = (size_t)m * 4, kb = (size_t)m;
+  CallScratch scratch;
+  int rc = scratch.take(c, align(xb) + align(tb) + align(kb) + 256, "qbc_proposal_gradient");
   if (rc) return rc;
-  float* dt = nullptr;
-  int8_t* dk = nullptr;
-  float* dl = nullptr;
-  cudaError_t e = cudaMalloc(&dt, (size_t)m * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&dk, (size_t)m);
-  if (e == cudaSuccess) e = cudaMalloc(&dl, 4);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dt, t, (size_t)m * 4, cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dk, kind, (size_t)m, cudaMemcpyHostToDevice, c->stream);
-  if (e != cudaSuccess) rc = fail(QBC_E_CUDA, "qbc_proposal_gradient: %s", cudaGetErrorString(e));
-  if (!rc) rc = c->net.gradient(dx, dt, dk, m, dl, c->stream);
-  if (!rc) {
-    e = cudaMemcpyAsync(loss, dl, 4, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(grad, c->net.grad, (size_t)QBC_PROPOSAL_PARAMS * 4, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    if (e != cudaSuccess) rc = fail(QBC_E_CUDA, "qbc_proposal_gradient: %s", cudaGetErrorString(e));
+  char* p = static_cast<char*>(scratch.ptr);
+  float* dx = reinterpret_cast<float*>(p);
+  float* dt = reinterpret_cast<float*>(p + align(xb));
+  int8_t* dk = reinterpret_cast<int8_t*>(p + align(xb) + align(tb));
+  float* dl = reinterpret_cast<float*>(p + align(xb) + align(tb) + align(kb));
+  QBC_CUDA(cudaMemcpyAsync(dx, x, xb, cudaMemcpyHostToDevice, c->stream));
+  QBC_CUDA(cudaMemcpyAsync(dt, t, tb, cudaMemcpyHostToDevice, c->stream));
+  QBC_CUDA(cudaMemcpyAsync(dk, kind, kb, cudaMemcpyHostToDevice, c->stream));
+  const int64_t l0 = qbc::mlp::launches();
+  rc = c->net.gradient(dx, dt, dk, m, dl, c->stream);
+  c->launches += qbc::mlp::launches() - l0;
+  if (rc) {
+    cudaStreamSynchronize(c->stream);  // the copies read the caller's arrays
+    return rc;
   }
-  cudaFree(dx);
-  cudaFree(dt);
-  cudaFree(dk);
-  cudaFree(dl);
-  return rc;
+  QBC_CUDA(cudaMemcpyAsync(loss, dl, 4, cudaMemcpyDeviceToHost, c->stream));
+  QBC_CUDA(cudaMemcpyAsync(grad, c->net.grad, (size_t)QBC_PROPOSAL_PARAMS * 4, cudaMemcpyDeviceToHost, c->stream));
+  QBC_CUDA(cudaStreamSynchronize(c->stream));
+  return QBC_OK;
 }

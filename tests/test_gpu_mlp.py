@@ -134,3 +134,24 @@ def test_train_then_propose(ctx):
     ctx.proposal_clear()
     with pytest.raises(QbcError):
         ctx.proposal_train(steps=1)
+
+
+@pytest.mark.parametrize("m", [1, 5, 127, 128, 129, 19455, 19457, 40001])
+def test_gradient_tiles(ctx, m):
+    """Rows that end inside, at and past a 128-row tile, and more tiles than an
+    SM each; the same tolerances as above. Equal inputs give equal bits."""
+    from oracle import mlp_ref
+    p = mlp_ref.random_params(9)
+    ctx.proposal_set_params(p)
+    x, t, kind = _data(m, m)
+    kind[::7] = -1  # rows without a label count for nothing but the mean
+    loss, g = ctx.proposal_gradient(x, t, kind)
+    again, h = ctx.proposal_gradient(x, t, kind)
+    assert again == loss and np.array_equal(bits(g), bits(h))
+    rloss, rg, ref = mlp_ref.loss_and_grad(p, x, t, kind)
+    assert abs(loss - rloss) <= 5e-3 * abs(rloss)
+    _, _, off = mlp_ref.layout()
+    for i in range(8):
+        a, b = g[off[i]:off[i + 1]], rg[off[i]:off[i + 1]]
+        assert np.linalg.norm(a - b) <= 2e-2 * max(np.linalg.norm(b), 1e-12), i
+    np.testing.assert_allclose(ctx.proposal_eval(x), ref, rtol=0, atol=1e-2)
