@@ -21,9 +21,12 @@
 // bounds of an axis in one packed FMA, and a descent reads its own list back
 // from the stack as a pop does (with branches around both, a view took 4.2
 // ms; without, 3.9). 16 x 1080p of a 20M-point room: 68.8 -> 44.7 ms, 37.8
-// with the service phase of render.cuh lightened as well; 4M random rays
-// 5.7 -> 4.2 ms. 6 blocks of 128 threads per SM (79 registers); 7 (18 bytes
-// spilled) measured the same, 8 spill 94 bytes and take 1.6x.
+// with the service phase of render.cuh lightened as well, 32 with that phase
+// looked for every six steps and the list's bit arithmetic shortened (octet
+// bits carried in the t values' low bits); 4M random rays 5.7 -> 4.0 ms. 6
+// blocks of 128 threads per SM (80 registers); 7 (18 bytes spilled) measured
+// the same, 8 spill 94 bytes and take 1.6x. Prefetching the next node's
+// record cost 3 % of a frame and half as much again of random rays.
 //
 // Path. The corner of the current cube is held per axis as the float 1 + path
 // bits (bit 22 - k for level k), so fma(X, S, -S) is the exact coordinate, a
@@ -149,9 +152,11 @@ static __device__ __forceinline__ uint32_t list_exact(const Spot r, const uint32
 
 // Instrumented renders: the box words the filter reads at a node, counted as
 // Walker::step counts them (entries whose child exists).
-static __device__ __noinline__ uint32_t words_read(const int32_t* child, int32_t node, uint32_t pk, int n) {
+__device__ __forceinline__ uint32_t words_read(const int32_t* child, int32_t node, uint32_t pk, int n) {
   uint32_t nw = 0;
-  for (int i = 0; i < n; ++i) nw += __ldg(child + 8 * (size_t)(uint32_t)node + ((pk >> (5 * i)) & 7u)) > 0 ? 1u : 0u;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (i < n) nw += __ldg(child + 8 * (size_t)(uint32_t)node + ((pk >> (5 * i)) & 7u)) > 0 ? 1u : 0u;
   return nw;
 }
 
@@ -201,6 +206,7 @@ struct FastWalker {
   bool slow;                  // this cube lies below an ambiguous one (or the ray allows no boxes)
   bool oob;
   uint32_t vis_s, vis_d;
+  uint32_t words;  // INSTR: leaf-box words the lane's walks read (sc.box_words set)
   // proposal test (PROP only): above tdepth the walk takes only the first
   // entry towards the cell of path `target` (3 bits per level, root first);
   // no entries are left there, so pops stop at tdepth
@@ -278,7 +284,7 @@ struct FastWalker {
     return kRunning;
   }
 
-  static constexpr float kRelGuard = 2.3841858e-06f;  // 40 * 2^-24
+  static constexpr float kRelGuard = 2.8610229e-06f;  // 48 * 2^-24
 
   // After start(): whether a two-tree walk of this ray reads the dynamic
   // tree, i.e. FastWalker<true>::start would not give it mode bit 3.
@@ -330,24 +336,26 @@ struct FastWalker {
       const float gc = fminf(fminf(fabsf(tx - ty), fabsf(ty - tz)), fabsf(tz - tx));
       const float lim = __fmaf_rn(t1, kRelGuard, __fmaf_rn(8.0f * lv2, guard, guard));
       exact = slow | !(fminf(fminf(ga, gb), gc) > lim);
-      // planes crossed inside the cube, in order: t with the axis in its two
-      // lowest bits, +inf for the others
+      // planes not yet crossed at the entry, in order of t; those past t1 are
+      // crossed outside. A t's three lowest bits hold its plane's octet bit.
       const bool bx = tx < t0, by = ty < t0, bz = tz < t0;
-      const float kx = (bx | !(tx < t1)) ? kInf : __uint_as_float(__float_as_uint(tx) & ~3u);
-      const float ky = (by | !(ty < t1)) ? kInf : __uint_as_float((__float_as_uint(ty) & ~3u) | 1u);
-      const float kz = (bz | !(tz < t1)) ? kInf : __uint_as_float((__float_as_uint(tz) & ~3u) | 2u);
+      const float kx = bx ? kInf : __uint_as_float((__float_as_uint(tx) & ~7u) | 1u);
+      const float ky = by ? kInf : __uint_as_float((__float_as_uint(ty) & ~7u) | 2u);
+      const float kz = bz ? kInf : __uint_as_float((__float_as_uint(tz) & ~7u) | 4u);
       const float m1 = fminf(kx, ky), m2 = fmaxf(kx, ky);
       const float k1 = fminf(m1, kz), m3 = fmaxf(m1, kz);
       const float k2 = fminf(m2, m3), k3 = fmaxf(m2, m3);
-      const uint32_t a1 = __float_as_uint(k1) & 3u, a2 = __float_as_uint(k2) & 3u, a3 = __float_as_uint(k3) & 3u;
+      const uint32_t b1 = __float_as_uint(k1), b2 = __float_as_uint(k2), b3 = __float_as_uint(k3);
       o[0] = ((bx ? 1u : 0u) | (by ? 2u : 0u) | (bz ? 4u : 0u)) ^ ((mode >> 4) & 7u);
-      o[1] = o[0] ^ (1u << a1);
-      o[2] = o[1] ^ (1u << a2);
-      o[3] = o[2] ^ (1u << a3);
-      v[1] = k1 < kInf;
-      v[2] = k2 < kInf;
-      v[3] = k3 < kInf;
-      pk = (((o[3] + 8u * a3) * 32u + (o[2] + 8u * a2)) * 32u + (o[1] + 8u * a1)) * 32u + (o[0] + 24u);
+      o[1] = o[0] ^ (b1 & 7u);
+      o[2] = o[1] ^ (b2 & 7u);
+      o[3] = o[2] ^ (b3 & 7u);
+      v[1] = k1 < t1;
+      v[2] = k2 < t1;
+      v[3] = k3 < t1;
+      // (octet bits 1, 2, 4 to sources 0, 1, 2)
+      pk = (((o[3] | ((b3 << 2) & 24u)) * 32u + (o[2] | ((b2 << 2) & 24u))) * 32u + (o[1] | ((b1 << 2) & 24u))) * 32u +
+           (o[0] + 24u);
     }
     if (__builtin_expect(exact, 0)) {
       pk = list_exact(spot(dir(), s), st.base, st.stride, kWords);
@@ -400,22 +408,23 @@ struct FastWalker {
       }
       const float2 tx = unpair(fma2(qx, u2x, cx)), ty = unpair(fma2(qy, u2y, cy)), tz = unpair(fma2(qz, u2z, cz));
       const float tn = fmaxf(fmaxf(tx.x, ty.x), tz.x), tf = fminf(fminf(tx.y, ty.y), tz.y);
-      return (tn <= tf) & (tf >= 0.0f);
+      // (a box behind the origin: listed cubes are not, so INSTR alone asks)
+      return (tn <= tf) & (!INSTR | (tf >= 0.0f));
     };
     // entries of a tree's node: the children with leaves (an empty child's
-    // record says so) whose box the ray meets; the deepest level's children
-    // are leaf cells, which every listed entry meets. All four records are
-    // read and tested, listed or not: they are in two sectors anyhow, and the
-    // lanes of a warp nearly always list four between them.
+    // record says so) whose box the ray meets (the deepest level's children
+    // are leaf cells, their boxes whole: every listed entry meets them). All
+    // four are tested, listed or not: the lanes of a warp nearly always list
+    // four between them. Only the listed are read: reading all four cost
+    // incoherent rays the record's other sector (4M rays 4.34 ms, 4.02 so).
     auto filter = [&](const DevTree& t, int32_t node) {
       const uint2* rec = reinterpret_cast<const uint2*>(t.cbox) + (size_t)(uint32_t)node * 8;
-      const bool any = level + 1 == t.box_depth;
       uint2 r[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) r[i] = __ldg(rec + o[i]);
+      for (int i = 0; i < 4; ++i) r[i] = v[i] ? __ldg(rec + o[i]) : make_uint2(kEmptyBox, 0u);
       uint32_t keep = 0u;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) keep |= (v[i] & (r[i].x != kEmptyBox) & (any | meets(r[i], o[i]))) ? 1u << i : 0u;
+      for (int i = 0; i < 4; ++i) keep |= ((r[i].x != kEmptyBox) & meets(r[i], o[i])) ? 1u << i : 0u;
       if (__builtin_expect(!geo, 0)) {  // the shader's own test (octree_fsh.c:313-317)
         const int32_t* c = reinterpret_cast<const int32_t*>(t.child) + 8 * (size_t)(uint32_t)node;
         keep = 0u;
@@ -430,14 +439,10 @@ struct FastWalker {
     if (DYN && has_d) kd = filter(sc.tree[1], nd);
     if (INSTR && sc.box_words) {
       const int n = 1 + (int)v[1] + (int)v[2] + (int)v[3];
-      uint32_t nw = 0u;
       if (geo && has_s && level + 1 < sc.tree[0].box_depth)
-        nw = words_read(reinterpret_cast<const int32_t*>(sc.tree[0].child), ns, pk, n);
+        words += words_read(reinterpret_cast<const int32_t*>(sc.tree[0].child), ns, pk, n);
       if (DYN && geo && has_d && level + 1 < sc.tree[1].box_depth)
-        nw += words_read(reinterpret_cast<const int32_t*>(sc.tree[1].child), nd, pk, n);
-      const unsigned am = __activemask();
-      const unsigned tot = __reduce_add_sync(am, nw);
-      if ((int)(threadIdx.x & 31u) == __ffs((int)am) - 1) atomicAdd(sc.box_words, (unsigned long long)tot);
+        words += words_read(reinterpret_cast<const int32_t*>(sc.tree[1].child), nd, pk, n);
     }
     // ---- take the next entry (octree_fsh.c:334-375) ----
     // The list goes to the stack and the nearest level with entries left is
