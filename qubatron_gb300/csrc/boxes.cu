@@ -28,7 +28,10 @@
 // after every level before). A node's children are neighbours in the order,
 // so their boxes are read in one run, and a level's boxes and records are
 // made in one kernel. 2.6M nodes of a 1M-point floor: 1.1 ms of kernels, 13
-// waits and five allocations before; 0.47 ms of kernels now.
+// waits and five allocations before; 0.47 ms of kernels then, 0.41 with the
+// order's positions reserved per block and a node's boxes read together. What
+// is left: the 64-byte records and 32-byte blocks of a level lie scattered
+// (0.3M-0.6M nodes take 20-40 us), and 36 launches, most of small levels.
 
 #include <cuda_runtime.h>
 
@@ -44,6 +47,7 @@ using qbc::fail;
 namespace qbc {
 namespace {
 
+constexpr int kThreads = 256;
 constexpr int kLevels = QBC_MAX_LEVEL + 1;  // levels expanded: nodes of a deeper one rule the boxes out
 
 struct Counts {
@@ -61,18 +65,22 @@ __device__ __forceinline__ void level_range(const Counts* c, int L, int64_t* b, 
 
 // Children of the nodes of level L appended to the order after them, each
 // with its position in pos; a node's first child's position to `first`. One
-// counter update per warp and pass: each lane takes its node's children, the
-// warp reserves their total at once.
-__global__ void expand_kernel(const int4* __restrict__ child, int64_t n, int32_t* __restrict__ order,
-                              int32_t* __restrict__ pos, int32_t* __restrict__ first, Counts* counts, int L) {
+// counter update per block and pass: each thread takes its node's children,
+// the block reserves their total at once (one update per warp: 38 us for a
+// level of 0.6M nodes, the updates of one address in turn; 25 so).
+__global__ void __launch_bounds__(kThreads) expand_kernel(const int4* __restrict__ child, int64_t n,
+                                                          int32_t* __restrict__ order, int32_t* __restrict__ pos,
+                                                          int32_t* __restrict__ first, Counts* counts, int L) {
+  __shared__ unsigned warp_total[kThreads / 32];
+  __shared__ unsigned long long reserved;
   int64_t in_b, in_e;
   level_range(counts, L, &in_b, &in_e);
   if (in_e > n) return;  // not a tree, detected on the host
-  const int lane = threadIdx.x & 31;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  // the loop's trip count is the same for the whole warp (ballots below)
-  for (int64_t j0 = in_b + (blockIdx.x * (int64_t)blockDim.x + threadIdx.x - lane); j0 < in_e; j0 += stride) {
-    const int64_t j = j0 + lane;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t stride = (int64_t)gridDim.x * kThreads;
+  // the loop's trip count is the same for the whole block (barriers below)
+  for (int64_t j0 = in_b + blockIdx.x * (int64_t)kThreads; j0 < in_e; j0 += stride) {
+    const int64_t j = j0 + tid;
     int32_t c[8];
     uint32_t take = 0;
     bool outside = false;
@@ -86,6 +94,7 @@ __global__ void expand_kernel(const int4* __restrict__ child, int64_t n, int32_t
         outside |= c[o] != 0 && !(c[o] > 0 && c[o] < n);
       }
     }
+    if (__any_sync(0xFFFFFFFFu, outside) && lane == 0) counts->bad = 1u;
     const unsigned mine = (unsigned)__popc(take);
     unsigned incl = mine;
 #pragma unroll
@@ -93,11 +102,17 @@ __global__ void expand_kernel(const int4* __restrict__ child, int64_t n, int32_t
       const unsigned v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
       if (lane >= o) incl += v;
     }
-    unsigned long long base = 0;
-    if (lane == 31 && incl) base = atomicAdd(&counts->level[L + 1], (unsigned long long)incl);
-    if (__any_sync(0xFFFFFFFFu, outside) && lane == 0) counts->bad = 1u;
-    base = __shfl_sync(0xFFFFFFFFu, base, 31);
-    int64_t k = in_e + (int64_t)base + (incl - mine);
+    if (lane == 31) warp_total[warp] = incl;
+    __syncthreads();
+    unsigned before = incl - mine, total = 0;
+#pragma unroll
+    for (int k = 0; k < kThreads / 32; ++k) {
+      if (k < warp) before += warp_total[k];
+      total += warp_total[k];
+    }
+    if (tid == 0) reserved = total ? atomicAdd(&counts->level[L + 1], (unsigned long long)total) : 0ull;
+    __syncthreads();
+    int64_t k = in_e + (int64_t)reserved + before;
     if (j < in_e) first[j] = (int32_t)min(k, n);
 #pragma unroll
     for (int o = 0; o < 8; ++o) {
@@ -125,32 +140,38 @@ __global__ void unique_kernel(const int32_t* __restrict__ order, const int32_t* 
 
 // Boxes in leaf cells of the nodes of level L, by position (children done),
 // and their records.
-__global__ void box_level_kernel(const int4* __restrict__ child, int64_t n, const int32_t* __restrict__ order,
-                                 const int32_t* __restrict__ first, const Counts* counts, int L,
-                                 uint4* __restrict__ box, uint4* __restrict__ rec) {
+__global__ void __launch_bounds__(kThreads)
+    box_level_kernel(const int4* __restrict__ child, int64_t n, const int32_t* __restrict__ order,
+                     const int32_t* __restrict__ first, const Counts* counts, int L, uint4* __restrict__ box,
+                     uint4* __restrict__ rec) {
   int64_t b, e, all_b, all_e;
   level_range(counts, L, &b, &e);
   level_range(counts, kLevels, &all_b, &all_e);
   if (counts->bad || all_e > n || all_b < all_e) return;  // no boxes
   int depth = L;
   while (depth + 1 <= kLevels && counts->level[depth + 1] > 0) ++depth;
+  if (L == depth) return;  // leaf cells: their box is their own cell
+  const bool last = L + 1 == depth;
   const int sh = depth - L - 1;  // a child's edge: 2^sh leaf cells
   for (int64_t j = b + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < e; j += (int64_t)gridDim.x * blockDim.x) {
-    if (L == depth) {
-      box[j] = make_uint4(0u, 0u, 0u, 0u);  // its own cell
-      continue;
-    }
     const int32_t node = order[j];
     int32_t c[8];
     load_children(child, node, c);
-    int64_t k = first[j];
+    const int64_t k = first[j];
+    // all children's boxes are read before the first is used (they depend on
+    // nothing but their number)
+    uint4 raw[8];
+    int m = 0;
+#pragma unroll
+    for (int o = 0; o < 8; ++o)
+      if (c[o] > 0 && c[o] < n) raw[o] = last ? make_uint4(0u, 0u, 0u, 0u) : box[k + m++];
     CellBox u = no_box();
     uint2 w[8];
 #pragma unroll
     for (int o = 0; o < 8; ++o) {
       w[o] = empty_word();
       if (!(c[o] > 0 && c[o] < n)) continue;
-      const CellBox v = unpack_box(box[k++]);
+      const CellBox v = unpack_box(raw[o]);
       if (v.lo[0] > v.hi[0]) continue;  // no leaves below
       w[o] = record_word(v, sh);
       add_box(u, v, o, sh);
@@ -185,13 +206,13 @@ int build_child_boxes(const int32_t* child, int64_t n, uint32_t* rec, void* scra
   // blocks of a level's kernel: the level holds at most min(n, 8^L) nodes
   auto blocks_of = [&](int L) {
     const int64_t most = L >= 10 ? n : std::min<int64_t>(n, int64_t(1) << (3 * L));
-    return (unsigned)std::min<int64_t>(grid, (most + 255) / 256);
+    return (unsigned)std::min<int64_t>(grid, (most + kThreads - 1) / kThreads);
   };
   for (int L = 0; L < kLevels; ++L)
-    expand_kernel<<<blocks_of(L), 256, 0, stream>>>(blocks, n, order, pos, first, counts, L);
-  unique_kernel<<<blocks_of(kLevels), 256, 0, stream>>>(order, pos, n, counts);
+    expand_kernel<<<blocks_of(L), kThreads, 0, stream>>>(blocks, n, order, pos, first, counts, L);
+  unique_kernel<<<blocks_of(kLevels), kThreads, 0, stream>>>(order, pos, n, counts);
   for (int L = kLevels - 1; L >= 0; --L)
-    box_level_kernel<<<blocks_of(L), 256, 0, stream>>>(blocks, n, order, first, counts, L, box, records);
+    box_level_kernel<<<blocks_of(L), kThreads, 0, stream>>>(blocks, n, order, first, counts, L, box, records);
   *launches += 2 * kLevels + 1;
   Counts h;
   e = cudaMemcpyAsync(&h, counts, sizeof(h), cudaMemcpyDeviceToHost, stream);
