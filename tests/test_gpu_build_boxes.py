@@ -53,6 +53,19 @@ def test_built_tree_and_boxes(oracle, n, levels, order):
                     assert np.array_equal(got[k], want[k]), k
 
 
+@pytest.mark.parametrize("n,levels", [(262143, 12), (262144, 5), (262144, 12), (300001, 9)])
+def test_large_dynamic_tree(n, levels):
+    """Around the size from which a few points go ahead of the others."""
+    import qubatron_gb300 as qb
+    p = _points(n, levels, np.random.default_rng(n), "shuffled")
+    p[-1000:] = p[:1000]  # first made by the points that go ahead, and met last
+    nodes = qb.build_octree(p, S, levels)
+    with qb.OctreeGLC(0) as ctx:
+        for _ in range(2):
+            assert ctx.build_tree(True, p, S, levels, first_index=0) == nodes.shape[0]
+            assert np.array_equal(ctx.download_tree(True), nodes)
+
+
 @pytest.mark.parametrize("kind", ["whole", "stubs", "twice", "outside", "root"])
 @pytest.mark.parametrize("n,levels", [(1, 3), (40, 1), (700, 8), (5000, 12)])
 def test_uploaded_boxes(oracle, kind, n, levels):
