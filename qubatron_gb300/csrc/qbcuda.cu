@@ -1215,9 +1215,16 @@ int launch_rays(qbc_ctx* c, const qbc::RayJob& job, size_t smem) {
   int per_sm = 0;
   QBC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, qbc::kThreads, smem));
   if (per_sm < 1) return fail(QBC_E_STATE, "rays_kernel: no block fits on an SM with %zu B shared memory", smem);
+  const int64_t resident = (int64_t)per_sm * c->sm_count;
+  // fewer rays than lanes: the rays far apart, so that each has lanes beside
+  // it that take parts of its walk
+  qbc::RayJob spread = job;
+  spread.spread = 0;
+  if (WALK != qbc::kWalkExact)
+    while (spread.spread < 5 && (job.n << (spread.spread + 1)) <= resident * qbc::kThreads) ++spread.spread;
   const int64_t blocks = std::max<int64_t>(
-      1, std::min<int64_t>((int64_t)per_sm * c->sm_count, (job.n + qbc::kThreads - 1) / qbc::kThreads));
-  kern<<<(unsigned)blocks, qbc::kThreads, smem, c->stream>>>(device_scene(c), job);
+      1, std::min<int64_t>(resident, ((job.n << spread.spread) + qbc::kThreads - 1) / qbc::kThreads));
+  kern<<<(unsigned)blocks, qbc::kThreads, smem, c->stream>>>(device_scene(c), spread);
   QBC_CUDA(cudaGetLastError());
   ++c->launches;
   return QBC_OK;

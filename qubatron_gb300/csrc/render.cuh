@@ -14,6 +14,7 @@
 
 #include "qbc_internal.h"
 #include "qbcuda.h"
+#include "share.cuh"
 #include "walker_fast.cuh"
 
 namespace qbc {
@@ -729,9 +730,11 @@ constexpr int kServiceMinDefault = 4;
 // after 6, 33.2 after 8; 1200x800 of a 5M-point room 1.21, 1.19, 1.16, 1.16,
 // 1.15, 1.15; the shortest walks (a small floor) gain nothing past 6.
 constexpr int kStepsPerLook = 6;
-// The same for ray queries: 1000 rays 201 us after every step, 191 after 4;
-// 4M random rays 4.44 and 4.35 ms.
-constexpr int kRaySteps = 4;
+// The same for ray queries, between two rounds of share_walks() at the end.
+// 4M random rays: 4.10 ms with 2 steps, 4.07 with 4, 4.02 with 8. Fewer rays
+// than lanes share from the start, and sooner is better there: 1000 rays 130
+// us a call with 2 steps, 139 with 4, 143 with 8 (188 without sharing).
+constexpr int kRaySteps = 8, kSpreadSteps = 2;
 
 // MODE kFused: every pixel's primary ray, shadow ray, shading and flare.
 // MODE kPrimaryPass: primary rays only; shaded and flare pixels go to the
@@ -987,6 +990,7 @@ struct RayJob {
   float4 bc;
   int32_t maxlevel;
   int32_t service_min;  // waiting lanes that start a service (1..32)
+  int32_t spread;       // one lane in 2^spread takes rays (0..5)
   qbc_ray_hits o;
 };
 
@@ -994,27 +998,49 @@ struct RayJob {
 // lane walks a sequence of rays (grid stride); a lane whose ray ended waits
 // until service_min lanes of its warp wait (or none runs), then they write
 // their results and start their next rays together, and the warp votes on
-// the division by reciprocals for the rays now running.
+// the division by reciprocals for the rays now running. Lanes without a ray
+// left share the others' walks (share.cuh; not where the walk is the
+// shader's own arithmetic, which keeps its entry points on the stack).
 template <bool EXACT, bool DYN, int WALK>
-__global__ void __launch_bounds__(kThreads) rays_kernel(DevScene sc, const __grid_constant__ RayJob job) {
+__global__ void __launch_bounds__(kThreads, WALK == kWalkFast ? 6 : 1) rays_kernel(DevScene sc, const __grid_constant__ RayJob job) {
   extern __shared__ uint32_t smem[];
   Stack st{smem + threadIdx.x, kThreads};
   WalkerOf<EXACT, DYN, false, WALK> w;
-  const int64_t stride = (int64_t)gridDim.x * kThreads;
+  const int64_t stride = (int64_t)gridDim.x * kThreads >> job.spread;
   int64_t i = blockIdx.x * (int64_t)kThreads + threadIdx.x;  // the lane's current ray
+  i = (i & ((1 << job.spread) - 1)) != 0 ? job.n : i >> job.spread;
   int r = kMiss;
   bool running = false, ended = false;  // ended: ray i is done and not yet written
   bool fast = false;                    // warp-uniform
-  auto ray_dir = [&] { return make_float3(job.dir[3 * i], job.dir[3 * i + 1], job.dir[3 * i + 2]); };
-  // warp-uniform: lanes without a ray left, which wait for nothing (counted
-  // as waiting, they had a warp at its end serve after every step: 1000 rays
-  // 244 us instead of 203)
-  int none = 0;
+  auto ray_dir = [&] {
+    const int64_t j = i < 0 ? -1 - i : i;  // (a lane that helps with ray j has i = -1 - j)
+    return make_float3(job.dir[3 * j], job.dir[3 * j + 1], job.dir[3 * j + 2]);
+  };
+  int none = 0;                 // warp-uniform: lanes without a ray of their own left; they wait for nothing
+  int serve = job.service_min;  // warp-uniform: waiting lanes that start a service
   if constexpr (WALK == kWalkFastInstr) w.words = 0u;
+  constexpr bool kShare = WALK != kWalkExact;
+  __shared__ int chain[kShare ? kThreads : 1];  // share_walks()'s next
+  if constexpr (kShare) chain[threadIdx.x] = kNoLane;
+  uint2 behind = make_uint2(0u, 0u);            // ... and behind
   for (;;) {
+    if constexpr (kShare) {
+      if (none) {
+        int kind = i < 0 ? kLaneHelper : (i < job.n ? kLaneOwner : kLaneFree);
+        int next = chain[threadIdx.x];
+        share_walks(w, st, job.maxlevel, kind, running, r, next, behind, [&](int src, bool mine) {
+          const int64_t ray = __shfl_sync(0xFFFFFFFFu, i, src);
+          if (mine) i = ray < 0 ? ray : -1 - ray;
+        });
+        if (kind == kLaneFree) i = job.n;
+        ended = kind == kLaneOwner && !running;
+        chain[threadIdx.x] = next;
+      }
+    }
     const unsigned run = __ballot_sync(0xFFFFFFFFu, running);
-    if (run == 0u || 32 - none - __popc(run) >= job.service_min) {
-      if (!running) {
+    const unsigned wait = __ballot_sync(0xFFFFFFFFu, !running && (none == 0 || (i >= 0 && i < job.n)));
+    if (run == 0u || __popc(wait) >= serve) {
+      if (!running && i >= 0) {
         for (;;) {
           if (ended) {
             int32_t ms = -1, md = -1, ls = -1, ld = -1;
@@ -1049,12 +1075,14 @@ __global__ void __launch_bounds__(kThreads) rays_kernel(DevScene sc, const __gri
           ended = true;  // written on the next pass of this loop
         }
       }
-      none = 32 - __popc(__ballot_sync(0xFFFFFFFFu, running));  // (every lane with a ray left runs now)
+      none = __popc(__ballot_sync(0xFFFFFFFFu, i < 0 || i >= job.n));
       if (none == 32) break;
+      // few rays left: each is written, and its lane goes on, without a wait
+      if (none) serve = min(job.service_min, max(1, (32 - none) >> 3));
       if constexpr (EXACT && WALK == kWalkExact) fast = __all_sync(0xFFFFFFFFu, !running || (w.mode & 1u));
     }
 #pragma unroll 1
-    for (int k = 0; k < kRaySteps; ++k) {
+    for (int k = job.spread ? kSpreadSteps : kRaySteps; k > 0; --k) {
       if (running) {
         if constexpr (WALK == kWalkExact) r = w.step(sc, job.maxlevel, job.bc, st, fast);
         else r = w.step(sc, job.maxlevel, job.bc, st, ray_dir);

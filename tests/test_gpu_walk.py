@@ -121,3 +121,31 @@ def test_bytes_alone(oracle, scene, shoot):
     with qb.OctreeGLC(0) as ctx:
         upload_scene(ctx, scene.nodes, col, nrm)
         assert np.array_equal(ctx.render_host([v], ("rgba8",))[0]["rgba8"], ref["rgba8"])
+
+
+@pytest.mark.parametrize("two_trees", [False, True])
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 129, 1000, 3649, 20_000])
+def test_few_rays(oracle, scene, character, n, two_trees):
+    """So few rays that lanes without one take parts of the others' walks:
+    results and visit counts are those of one lane's walk."""
+    import qubatron_gb300 as qb
+    from qubatron_gb300 import _lib as L
+    rng = np.random.default_rng(n)
+    pos = rng.uniform(0.05 * S, 0.95 * S, (n, 3)).astype(np.float32)
+    d = rng.normal(size=(n, 3)).astype(np.float32)
+    d[::3] *= np.float32([1.0, 1e-3, 1.0])  # along the floor: long walks
+    lp, ld = _rays("lattice", n, rng)
+    pos[::5], d[::5] = lp[::5], ld[::5]
+    dyn = character if two_trees else (None, None, None)
+    with qb.OctreeGLC(0) as ctx:
+        upload_scene(ctx, scene.nodes, scene.colors, scene.normals, *dyn)
+        plain, counted = _trace(ctx, pos, d, False), _trace(ctx, pos, d, True)
+        ctx.set_option(L.OPT_BOX_PRUNE, 0)
+        shader = _trace(ctx, pos, d, True)
+    ref = oracle.trace_rays(oracle_scene(oracle, scene.nodes, scene.colors, scene.normals, *dyn, boxes=True), BASE,
+                            LEVELS, pos, d)
+    for k in ("status", "leaf", "model", "isp", "col", "nrm"):
+        assert np.array_equal(bits(plain[k]), bits(shader[k])), k
+        assert np.array_equal(bits(counted[k]), bits(shader[k])), k
+    for k in ("status", "leaf", "model", "visits"):
+        assert np.array_equal(counted[k], ref[k]), k
