@@ -52,6 +52,7 @@ struct qbc_ctx {
   size_t stage_bytes = 0;
   void* scratch = nullptr;  // ensure_scratch's
   size_t scratch_bytes = 0;
+  void* pinned = nullptr;  // host memory for small calls' copies (kPinnedMax bytes)
   unsigned int* queue = nullptr;  // global tile counter of the persistent render kernel
   // two-pass render: records, counters (queued, shade-pass next), statistics, per-pixel log
   uint32_t* rec = nullptr;
@@ -102,6 +103,10 @@ int check_device_errors(qbc_ctx* c);
 int dynamic_update(qbc_ctx* c, const qbc_dynamic_update* u);
 
 constexpr size_t kStageMax = size_t(256) << 20;
+// Calls with at most this many bytes copy through the context's pinned buffer
+// (ray queries on host arrays, 100 bytes a ray: 1000 rays 130 -> 76 us, 3000
+// 167 -> 129, 16384 230 -> 245: the copies in and out of the buffer).
+constexpr size_t kPinnedMax = size_t(512) << 10;
 
 inline int cuda_fail(cudaError_t e, const char* what) {
   return fail(QBC_E_CUDA, "%s: %s", what, cudaGetErrorString(e));

@@ -92,6 +92,7 @@ extern "C" int qbc_destroy(qbc_ctx* c) {
     cudaFree(c->model[t].nrm);
   }
   cudaFree(c->stage);
+  cudaFreeHost(c->pinned);
   cudaFree(c->scratch);
   cudaFree(c->queue);
   c->net.release();
@@ -1230,6 +1231,27 @@ int launch_rays(qbc_ctx* c, const qbc::RayJob& job, size_t smem) {
   return QBC_OK;
 }
 
+// Whether the host may read and write what p points to (null: nothing to do).
+static bool on_host(const void* p) {
+  if (!p) return true;
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeUnregistered || a.type == cudaMemoryTypeHost;
+}
+
+// The context's kPinnedMax bytes of pinned memory, made when first wanted;
+// null where there is none to be had.
+static void* pinned_buffer(qbc_ctx* c) {
+  if (!c->pinned && cudaMallocHost(&c->pinned, kPinnedMax) != cudaSuccess) {
+    cudaGetLastError();
+    c->pinned = nullptr;
+  }
+  return c->pinned;
+}
+
 extern "C" int qbc_trace_rays(qbc_ctx* c, const float* pos, const float* dir, int64_t n, const float basecube[4],
                               int maxlevel, const qbc_ray_hits* out, int on_device) {
   qbc::clear_error();
@@ -1257,6 +1279,8 @@ extern "C" int qbc_trace_rays(qbc_ctx* c, const float* pos, const float* dir, in
                         (void* const*)&out->isp,    (void* const*)&out->col,  (void* const*)&out->nrm,
                         (void* const*)&out->visits};
   void* dv[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+  char* packed = nullptr;  // pinned copy of the scratch: inputs, then outputs
+  size_t in_bytes = 0, all_bytes = 0;
   if (on_device) {
     job.pos = pos;
     job.dir = dir;
@@ -1278,8 +1302,20 @@ extern "C" int qbc_trace_rays(qbc_ctx* c, const float* pos, const float* dir, in
       dv[k] = base + off;
       off += ((size_t)n * bytes[k] + 255) & ~size_t(255);
     }
-    QBC_CUDA(cudaMemcpyAsync(dpos, pos, (size_t)n * 12, cudaMemcpyHostToDevice, c->stream));
-    QBC_CUDA(cudaMemcpyAsync(ddir, dir, (size_t)n * 12, cudaMemcpyHostToDevice, c->stream));
+    in_bytes = (size_t)((char*)ddir - base) + (size_t)n * 12;
+    all_bytes = off;
+    // Small calls: one copy each way through pinned memory (a copy from or to
+    // an array of the caller's costs some 10 us whatever its size).
+    bool host = all_bytes <= kPinnedMax && on_host(pos) && on_host(dir);
+    for (int k = 0; k < 7; ++k) host = host && on_host(*hs[k]);
+    if (host && (packed = (char*)pinned_buffer(c)) != nullptr) {
+      std::memcpy(packed, pos, (size_t)n * 12);
+      std::memcpy(packed + ((char*)ddir - base), dir, (size_t)n * 12);
+      QBC_CUDA(cudaMemcpyAsync(base, packed, in_bytes, cudaMemcpyHostToDevice, c->stream));
+    } else {
+      QBC_CUDA(cudaMemcpyAsync(dpos, pos, (size_t)n * 12, cudaMemcpyHostToDevice, c->stream));
+      QBC_CUDA(cudaMemcpyAsync(ddir, dir, (size_t)n * 12, cudaMemcpyHostToDevice, c->stream));
+    }
     job.pos = dpos;
     job.dir = ddir;
   }
@@ -1297,7 +1333,15 @@ extern "C" int qbc_trace_rays(qbc_ctx* c, const float* pos, const float* dir, in
   int rc = exact ? (dyn ? launch_rays<true, true>(c, job, smem) : launch_rays<true, false>(c, job, smem))
                  : (dyn ? launch_rays<false, true>(c, job, smem) : launch_rays<false, false>(c, job, smem));
   if (rc) return rc;
-  if (!on_device) {
+  if (packed) {
+    const size_t from = (in_bytes + 255) & ~size_t(255);  // the first output
+    if (all_bytes > from)
+      QBC_CUDA(cudaMemcpyAsync(packed + from, (char*)c->scratch + from, all_bytes - from, cudaMemcpyDeviceToHost,
+                               c->stream));
+    QBC_CUDA(cudaStreamSynchronize(c->stream));
+    for (int k = 0; k < 7; ++k)
+      if (*hs[k]) std::memcpy(*hs[k], packed + ((char*)dv[k] - (char*)c->scratch), (size_t)n * bytes[k]);
+  } else if (!on_device) {
     for (int k = 0; k < 7; ++k)
       if (*hs[k]) QBC_CUDA(cudaMemcpyAsync(*hs[k], dv[k], (size_t)n * bytes[k], cudaMemcpyDeviceToHost, c->stream));
     QBC_CUDA(cudaStreamSynchronize(c->stream));

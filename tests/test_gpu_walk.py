@@ -149,3 +149,22 @@ def test_few_rays(oracle, scene, character, n, two_trees):
         assert np.array_equal(bits(counted[k]), bits(shader[k])), k
     for k in ("status", "leaf", "model", "visits"):
         assert np.array_equal(counted[k], ref[k]), k
+
+
+@pytest.mark.parametrize("n", [1, 2, 5200, 5240, 5243, 5300])
+def test_host_outputs(scene, n):
+    """Any choice of outputs, around the size up to which they are copied
+    together (512 KB with all of them)."""
+    import qubatron_gb300 as qb
+    from qubatron_gb300 import _lib
+    pos, d = _rays("lattice", n, np.random.default_rng(n))
+    with qb.OctreeGLC(0) as ctx:
+        upload_scene(ctx, scene.nodes, scene.colors, scene.normals)
+        want = _trace(ctx, pos, d, True)
+        for names in (("status",), ("leaf", "isp"), ("visits", "model"), ("col", "nrm", "status"), ()):
+            got = {k: np.full_like(want[k], 77) for k in names}
+            h = _lib.RayHits(**{k: a.ctypes.data for k, a in got.items()})
+            _lib.check(ctx._lib.qbc_trace_rays(ctx.handle, C.c_void_p(pos.ctypes.data), C.c_void_p(d.ctypes.data), n,
+                                               (C.c_float * 4)(*BASE), LEVELS, C.byref(h), 0))
+            for k in names:
+                assert np.array_equal(bits(got[k]), bits(want[k])), (names, k)
