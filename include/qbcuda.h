@@ -580,8 +580,8 @@ int qbc_launch_count(qbc_ctx* ctx, int64_t* count);
  * GPU tree build into the context's static (tree 0) or dynamic (tree 1)
  * octree: the node array that inserting the n points in order into an empty
  * tree gives (octree_reset + octree_insert_point, octree.c:89-147, model
- * indices first_index + i), numbering included, built with sorts and prefix
- * sums instead of one walk per point. The result replaces the tree exactly
+ * indices first_index + i), numbering included, built with creator tables and
+ * prefix sums instead of one walk per point. The result replaces the tree exactly
  * as a whole-array qbc_upload of that array would. pnts is n float3 on the
  * host (on_device = 0) or on the context's GPU.
  */
