@@ -83,7 +83,22 @@ constexpr int64_t kPilot = 8192, kPilotMin = 262144;
 constexpr int kPilotLevel = 9;
 constexpr int kKeyGroups = 4;         // groups of 32 points a warp makes keys of at a time
 constexpr int kClimbThreads = 64;      // threads end at different levels: small blocks give their room back early
-constexpr int kScanThreads = 256, kScanPer = 8, kScanChunk = kScanThreads * kScanPer;
+// Points per chunk of the prefix sum and of the child blocks' writing: 8 a
+// thread, and 1 up to kScanFew points (still one pass over the chunk sums),
+// whose few chunks left most SMs idle and each warp a long run of blocks: 50k
+// points 50 us for the two kernels in 25 chunks, 13 in 196; a 50k-point
+// character skinned, built and drawn 798 -> 788 us.
+constexpr int kScanThreads = 256, kScanPer = 8;
+constexpr int64_t kScanFew = 262144;
+
+constexpr int64_t scan_chunks(int64_t n) {
+  const int64_t chunk = kScanThreads * (n <= kScanFew ? 1 : kScanPer);
+  return n <= 0 ? 1 : (n + chunk - 1) / chunk;
+}
+// ... of any build of at most n points.
+constexpr int64_t scan_chunks_most(int64_t n) {
+  return n <= kScanFew ? scan_chunks(n) : std::max(scan_chunks(n), scan_chunks(kScanFew));
+}
 
 __host__ __device__ constexpr int dense_offset(int l) {  // first entry of level l's prefix table
   return l <= 1 ? 0 : (l == 2 ? 8 : (l == 3 ? 72 : 584));
@@ -310,9 +325,10 @@ __device__ __forceinline__ int32_t made(const uint8_t* own, int64_t i, int64_t n
   return i < n ? max(levels + 1 - (int)own[i], 0) : 0;
 }
 
-// Prefix sum, pass 1: nodes made per chunk of kScanChunk points. With
+// Prefix sum, pass 1: nodes made per chunk of PER points a thread. With
 // creator tables the deepest level is resolved on the way (t_res; and the
 // entries of the level above reset, t_clr), as level_kernel does.
+template <int PER>
 __global__ void scan_chunks_kernel(uint8_t* __restrict__ own, const uint64_t* __restrict__ key, int64_t n, int levels,
                                    const uint32_t* __restrict__ slot, uint32_t* __restrict__ par,
                                    const uint32_t* __restrict__ t_res, uint32_t* __restrict__ t_clr,
@@ -321,8 +337,8 @@ __global__ void scan_chunks_kernel(uint8_t* __restrict__ own, const uint64_t* __
   const int64_t b = blockIdx.x;
   int32_t sum = 0;
 #pragma unroll
-  for (int k = 0; k < kScanPer; ++k) {
-    const int64_t i = b * kScanChunk + (int64_t)k * kScanThreads + threadIdx.x;
+  for (int k = 0; k < PER; ++k) {
+    const int64_t i = (b * PER + k) * kScanThreads + threadIdx.x;
     if (i >= n) break;
     int o = own[i];
     if (t_res) {
@@ -376,13 +392,14 @@ __global__ void scan_top_kernel(int32_t* __restrict__ blocksum, int64_t nb, int3
 // the nodes it makes. A warp takes 32 points at a time; their nodes are one
 // run of ids, and its lanes write that run's blocks (two lanes a block) in
 // order, whichever point a node belongs to.
+template <int PER>
 __global__ void spread_kernel(const uint8_t* __restrict__ own, const uint64_t* __restrict__ key, int64_t n, int levels,
                               const int32_t* __restrict__ blocksum, int32_t* __restrict__ base, int64_t first_index,
                               int4* __restrict__ child, int32_t* __restrict__ model, uint32_t* __restrict__ rec) {
-  constexpr int kWarps = kScanThreads / 32, kGroups = kScanChunk / kScanThreads;
+  constexpr int kWarps = kScanThreads / 32, kGroups = PER;
   __shared__ int32_t sh[kWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t p0 = (int64_t)blockIdx.x * kScanChunk + warp * (kScanChunk / kWarps);
+  const int64_t p0 = ((int64_t)blockIdx.x * kWarps + warp) * (32 * kGroups);
   int32_t incl[kGroups], sum = 0;
 #pragma unroll
   for (int g = 0; g < kGroups; ++g) {
@@ -618,7 +635,7 @@ int build_reserve(BuildScratch* s, int64_t n, int levels) {
     s->tab_points = m;
     s->dirty = true;  // emptied on the build's stream
   }
-  const int64_t nb = (n + kScanChunk - 1) / kScanChunk;
+  const int64_t nb = scan_chunks_most(n);
   if (s->blocks < nb || !s->blocksum) {
     s->blocks = 0;
     rc = grow_buf(&s->blocksum, 0, std::max<int64_t>(nb, 1), "block sums");
@@ -646,9 +663,9 @@ uint32_t* level_table(const BuildScratch* s, int l) { return s->tab[l % 3]; }
 // node count goes to *total.
 void count_nodes(int64_t n, int levels, const BuildScratch* s, bool sorted, int32_t* total, cudaStream_t stream,
                  int64_t* launches) {
-  const int64_t nb = std::max<int64_t>(1, (n + kScanChunk - 1) / kScanChunk);
+  const int64_t nb = scan_chunks(n);
   const bool tables = !sorted && levels > kDense;
-  scan_chunks_kernel<<<(unsigned)nb, kScanThreads, 0, stream>>>(
+  (n <= kScanFew ? scan_chunks_kernel<1> : scan_chunks_kernel<kScanPer>)<<<(unsigned)nb, kScanThreads, 0, stream>>>(
       s->own, s->key, n, levels, s->slot, s->par, tables ? level_table(s, levels) : nullptr,
       tables && levels - 1 > kDense ? level_table(s, levels - 1) : nullptr, s->blocksum);
   scan_top_kernel<<<1, 1024, 0, stream>>>(s->blocksum, nb, total);
@@ -660,9 +677,9 @@ void count_nodes(int64_t n, int levels, const BuildScratch* s, bool sorted, int3
 void write_tree(int64_t n, int levels, int64_t first_index, const BuildScratch* s, bool sorted, bool reset,
                 int64_t nodes, int32_t* child, int32_t* model, uint32_t* rec, cudaStream_t stream,
                 int64_t* launches) {
-  const int64_t nb = std::max<int64_t>(1, (n + kScanChunk - 1) / kScanChunk);
-  spread_kernel<<<(unsigned)nb, kScanThreads, 0, stream>>>(s->own, s->key, n, levels, s->blocksum, s->base,
-                                                           first_index, reinterpret_cast<int4*>(child), model, rec);
+  const int64_t nb = scan_chunks(n);
+  (n <= kScanFew ? spread_kernel<1> : spread_kernel<kScanPer>)<<<(unsigned)nb, kScanThreads, 0, stream>>>(
+      s->own, s->key, n, levels, s->blocksum, s->base, first_index, reinterpret_cast<int4*>(child), model, rec);
   ++*launches;
   if (n > 0 && levels > 0) {
     const int4* blocks = reinterpret_cast<const int4*>(child);
@@ -775,7 +792,7 @@ int build_tree_static(const float* d_pts, const int32_t* d_octets, int64_t n, fl
   BuildScratch s;
   Arena arena(stream);
   // per-point state in one allocation, its parts 256-byte aligned
-  const int64_t m = std::max<int64_t>(n, 1), nb = std::max<int64_t>((n + kScanChunk - 1) / kScanChunk, 1);
+  const int64_t m = std::max<int64_t>(n, 1), nb = scan_chunks(n);
   size_t off = 0;
   auto part = [&](size_t bytes) {
     const size_t at = off;

@@ -66,6 +66,18 @@ def test_large_dynamic_tree(n, levels):
             assert np.array_equal(ctx.download_tree(True), nodes)
 
 
+def test_dynamic_tree_of_changing_size():
+    """Scratch made for one size serves the smaller sizes, whose prefix sums
+    have more chunks (up to 262144 points)."""
+    import qubatron_gb300 as qb
+    p = _points(300001, 8, np.random.default_rng(1), "shuffled")
+    with qb.OctreeGLC(0) as ctx:
+        for n in (300001, 262144, 262145, 257, 256, 1, 200000):
+            nodes = qb.build_octree(p[:n], S, 8)
+            assert ctx.build_tree(True, p[:n], S, 8, first_index=0) == nodes.shape[0]
+            assert np.array_equal(ctx.download_tree(True), nodes), n
+
+
 @pytest.mark.parametrize("kind", ["whole", "stubs", "twice", "outside", "root"])
 @pytest.mark.parametrize("n,levels", [(1, 3), (40, 1), (700, 8), (5000, 12)])
 def test_uploaded_boxes(oracle, kind, n, levels):
