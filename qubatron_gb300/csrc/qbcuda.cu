@@ -1204,7 +1204,7 @@ int render_views_impl(qbc_ctx* c, const qbc_view* views, const qbc_outputs* outs
 }
 
 // Ray queries: one wave of resident blocks (lanes take rays by grid stride),
-// never more blocks than the rays need.
+// never more blocks than the rays, spread over the lanes, need.
 template <bool EXACT, bool DYN, int WALK = qbc::kWalkExact>
 int launch_rays(qbc_ctx* c, const qbc::RayJob& job, size_t smem) {
   if constexpr (EXACT && WALK == qbc::kWalkExact) {

@@ -7,7 +7,7 @@
 // cube. For almost every cube those comparisons follow from the ray's t at the
 // planes alone: the octet of the entry point is given by the planes crossed
 // before the entry t, and every plane crossed before the exit t starts the
-// next octet. list_fast() works on the t values, and first checks that no two
+// next octet. step() works on the t values, and first checks that no two
 // of the t values it compares are closer than the rounding errors, its own and
 // the shader's, could bridge (`guard`). Where two are, list_exact() does the
 // shader's arithmetic from the exact entry point, for this cube and the
