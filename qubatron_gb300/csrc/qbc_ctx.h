@@ -8,9 +8,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <bitset>
 #include <cstdint>
 #include <vector>
 
+#include "kernel_index.h"
 #include "mlp.h"
 #include "qbc_internal.h"
 #include "qbcuda.h"
@@ -72,7 +74,7 @@ struct qbc_ctx {
   bool fused_attr[2] = {false, false};  // dynamic shared memory set for the fused network kernels
   std::vector<qbc_graph*> graphs;       // captured frames, detached when the context goes
   int render_blocks[4] = {0, 0, 0, 0};  // resident blocks per SM of each render_kernel variant
-  uint64_t attr_done = 0;  // kernel variants whose shared-memory limit is set (bit per variant)
+  std::bitset<qbc::kKernels> attr_done;  // kernels whose shared-memory limit is set (kernel_index.h)
   int service_min = qbc::kServiceMinDefault;
   int tile_shift = 3;     // 8x4 warp tiles
   int blocks_per_sm = 0;  // render blocks per SM (0: as many as fit)

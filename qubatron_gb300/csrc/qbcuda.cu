@@ -881,10 +881,7 @@ bool instrumented(const qbc::Batch& b) {
   return false;
 }
 
-// Bit of a render kernel in qbc_ctx::attr_done.
-constexpr int kernel_variant(bool exact, bool dyn, int mode, bool prop, int walk) {
-  return (exact ? 1 : 0) + (dyn ? 2 : 0) + 4 * (mode + (prop ? 5 : 0)) + 24 * walk;
-}
+static_assert(qbc::kSplitFinish + 1 == qbc::kModeKinds && qbc::kWalkFastInstr + 1 == qbc::kWalkKinds, "kernel numbers");
 
 template <bool EXACT, bool DYN, int MODE, bool PROP, int WALK = qbc::kWalkExact>
 int launch_render(qbc_ctx* c, const qbc::Batch& b, size_t smem, const qbc::Wave& wave) {
@@ -898,10 +895,11 @@ int launch_render(qbc_ctx* c, const qbc::Batch& b, size_t smem, const qbc::Wave&
     }
   }
   auto kern = qbc::render_kernel<EXACT, DYN, MODE, PROP, WALK>;
-  const int variant = kernel_variant(EXACT, DYN, MODE, PROP, WALK);
-  if (!(c->attr_done & (1ull << variant))) {
+  static_assert(!PROP || MODE == qbc::kShadePass, "kernel numbers");
+  constexpr int variant = qbc::render_kernel_index(EXACT, DYN, MODE, PROP, WALK);
+  if (!c->attr_done[variant]) {
     QBC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-    c->attr_done |= 1ull << variant;
+    c->attr_done[variant] = true;
   }
   int per_sm = 0;
   QBC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, qbc::kThreads, smem));
@@ -928,10 +926,10 @@ int launch_render(qbc_ctx* c, const qbc::Batch& b, size_t smem, const qbc::Wave&
 template <bool EXACT, bool DYN>
 int launch_simple(qbc_ctx* c, const qbc::Batch& b, size_t smem) {
   auto kern = qbc::simple_kernel<EXACT, DYN>;
-  const int variant = 60 + (EXACT ? 1 : 0) + (DYN ? 2 : 0);
-  if (!(c->attr_done & (1ull << variant))) {
+  constexpr int variant = qbc::simple_kernel_index(EXACT, DYN);
+  if (!c->attr_done[variant]) {
     QBC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-    c->attr_done |= 1ull << variant;
+    c->attr_done[variant] = true;
   }
   const int64_t blocks = std::max<int64_t>(1, ((int64_t)b.tiles_total + 3) / 4);
   qbc::DevScene sc = device_scene(c);
@@ -1431,11 +1429,11 @@ namespace {
 // kernel's code under lazy module loading.
 template <bool EXACT, bool DYN, int WALK = qbc::kWalkExact>
 int fused_attr(qbc_ctx* c) {
-  const int variant = kernel_variant(EXACT, DYN, qbc::kFused, false, WALK);
-  if (!(c->attr_done & (1ull << variant))) {
+  constexpr int variant = qbc::render_kernel_index(EXACT, DYN, qbc::kFused, false, WALK);
+  if (!c->attr_done[variant]) {
     QBC_CUDA(cudaFuncSetAttribute(qbc::render_kernel<EXACT, DYN, qbc::kFused, false, WALK>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
-    c->attr_done |= 1ull << variant;
+    c->attr_done[variant] = true;
   }
   return QBC_OK;
 }
