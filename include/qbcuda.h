@@ -456,7 +456,9 @@ int qbc_graph_capture(qbc_ctx* ctx, const qbc_view* views, const qbc_outputs* de
  * update->bones (on the context's stream, or before the launch) and call
  * qbc_graph_launch. The update's arrays and sizes are held by the graph; the
  * dynamic tree's buffers are sized for the update's node bound, so replays
- * never reallocate. qbc_graph_update re-captures both parts.
+ * never reallocate. A larger build of the dynamic tree in between, which
+ * replaces the build's scratch, makes qbc_graph_launch fail like the changes
+ * above. qbc_graph_update re-captures both parts.
  */
 int qbc_graph_capture_dynamic(qbc_ctx* ctx, const qbc_dynamic_update* update, const qbc_view* views, const qbc_outputs* dev_outs, int n, const qbc_render_opts* opts, qbc_graph** graph);
 int qbc_graph_update(qbc_graph* graph, const qbc_view* views, int n);

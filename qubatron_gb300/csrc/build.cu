@@ -620,6 +620,7 @@ int build_reserve(BuildScratch* s, int64_t n, int levels) {
   const int64_t m = std::max<int64_t>(n, 1);
   if (s->points < n || !s->key) {
     s->points = 0;
+    ++s->generation;
     if (!rc) rc = grow_buf(&s->key, 0, m, "keys");
     if (!rc) rc = grow_buf(&s->par, 0, m, "parents");
     if (!rc) rc = grow_buf(&s->base, 0, m, "node ids");
@@ -630,6 +631,7 @@ int build_reserve(BuildScratch* s, int64_t n, int levels) {
   }
   if (levels > kDense && (s->tab_points < n || !s->tab[0])) {
     s->tab_points = 0;
+    ++s->generation;
     for (int t = 0; t < 3 && !rc; ++t) rc = grow_buf(&s->tab[t], 0, 8 * m, "creator tables");
     if (rc) return rc;
     s->tab_points = m;
@@ -638,18 +640,23 @@ int build_reserve(BuildScratch* s, int64_t n, int levels) {
   const int64_t nb = scan_chunks_most(n);
   if (s->blocks < nb || !s->blocksum) {
     s->blocks = 0;
+    ++s->generation;
     rc = grow_buf(&s->blocksum, 0, std::max<int64_t>(nb, 1), "block sums");
     if (rc) return rc;
     s->blocks = std::max<int64_t>(nb, 1);
   }
   if (s->box_nodes < nodes || !s->box) {
     s->box_nodes = 0;
+    ++s->generation;
     rc = grow_buf(&s->box, 0, nodes, "leaf boxes");
     if (!rc) rc = grow_buf(&s->arrived, 0, nodes / 8 + 1, "arrivals");
     if (rc) return rc;
     s->box_nodes = nodes;
   }
-  if (!s->dense) rc = grow_buf(&s->dense, 0, kDenseEntries, "prefix tables");
+  if (!s->dense) {
+    ++s->generation;
+    rc = grow_buf(&s->dense, 0, kDenseEntries, "prefix tables");
+  }
   return rc;
 }
 

@@ -37,6 +37,11 @@ struct FrameSignature {
   int32_t persistent;
   int32_t proposal_level;
   int32_t split_trees;
+  // of a frame with a dynamic update: what its build writes to besides the
+  // tree itself (the scratch by its generation; the leaf-box records, which
+  // the scene names only where the walk uses them)
+  uint64_t build_scratch;
+  const void* build_records;
 };
 
 bool same_signature(const FrameSignature& a, const FrameSignature& b) {
@@ -51,10 +56,11 @@ bool same_signature(const FrameSignature& a, const FrameSignature& b) {
          a.net_w == b.net_w && a.net_b == b.net_b && a.stream == b.stream && a.service_min == b.service_min &&
          a.proposal_gate == b.proposal_gate && a.tile_shift == b.tile_shift && a.blocks_per_sm == b.blocks_per_sm &&
          a.proposal_count == b.proposal_count && a.persistent == b.persistent &&
-         a.proposal_level == b.proposal_level && a.split_trees == b.split_trees;
+         a.proposal_level == b.proposal_level && a.split_trees == b.split_trees &&
+         a.build_scratch == b.build_scratch && a.build_records == b.build_records;
 }
 
-FrameSignature frame_signature(const qbc_ctx* c) {
+FrameSignature frame_signature(const qbc_ctx* c, bool has_update) {
   FrameSignature f;
   f.scene = device_scene(c);
   f.rec = c->rec;
@@ -72,6 +78,8 @@ FrameSignature frame_signature(const qbc_ctx* c) {
   f.persistent = c->persistent;
   f.proposal_level = c->proposal_level;
   f.split_trees = c->split_trees;
+  f.build_scratch = has_update ? c->build.generation : 0;
+  f.build_records = has_update ? c->tree[1].cbox : nullptr;
   return f;
 }
 
@@ -171,7 +179,7 @@ int capture_impl(qbc_ctx* c, const qbc_dynamic_update* update, const qbc_view* v
     g->opts = *opts;
     g->has_opts = true;
   }
-  g->sig = frame_signature(c);
+  g->sig = frame_signature(c, g->has_update);
   rc = capture_frame(g.get(), views, &g->graph);
   if (rc) return rc;
   cudaError_t e = cudaGraphInstantiate(&g->exec, g->graph, 0);
@@ -214,7 +222,7 @@ extern "C" int qbc_graph_update(qbc_graph* g, const qbc_view* views, int n) {
   // leaf boxes rebuilt outside the capture (that allocates and synchronises)
   int brc = ensure_boxes(c);
   if (brc) return brc;
-  g->sig = frame_signature(c);
+  g->sig = frame_signature(c, g->has_update);
   cudaGraph_t fresh = nullptr;
   int rc = capture_frame(g, views, &fresh);
   if (rc) return rc;
@@ -242,7 +250,7 @@ extern "C" int qbc_graph_launch(qbc_graph* g) {
   if (!g) return fail(QBC_E_ARG, "qbc_graph_launch: null graph");
   if (!g->ctx || !g->exec) return fail(QBC_E_STATE, "qbc_graph_launch: the graph's context was destroyed");
   qbc_ctx* c = g->ctx;
-  if (!same_signature(frame_signature(c), g->sig))
+  if (!same_signature(frame_signature(c, g->has_update), g->sig))
     return fail(QBC_E_STATE, "qbc_graph_launch: scene, buffers, stream or options changed since the capture "
                              "(qbc_graph_update re-captures)");
   QBC_CUDA(cudaSetDevice(c->device));

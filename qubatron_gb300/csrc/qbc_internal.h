@@ -48,6 +48,7 @@ struct BuildScratch {
   uint4* box = nullptr;      // boxes of nodes with siblings, 6 x 21 bits
   uint32_t* arrived = nullptr;  // children done, 4 bits a node
   bool dirty = false;        // tables new, or left by a build that stopped midway: to be emptied
+  uint64_t generation = 0;   // raised whenever an array is replaced: captured builds hold their addresses
 };
 
 // Nodes a build of n points at `levels` can make: 1 + sum over levels l of
