@@ -222,7 +222,7 @@ extern "C" int qbc_graph_update(qbc_graph* g, const qbc_view* views, int n) {
   // leaf boxes rebuilt outside the capture (that allocates and synchronises)
   int brc = ensure_boxes(c);
   if (brc) return brc;
-  g->sig = frame_signature(c, g->has_update);
+  const FrameSignature sig = frame_signature(c, g->has_update);
   cudaGraph_t fresh = nullptr;
   int rc = capture_frame(g, views, &fresh);
   if (rc) return rc;
@@ -241,6 +241,7 @@ extern "C" int qbc_graph_update(qbc_graph* g, const qbc_view* views, int n) {
   }
   cudaGraphDestroy(g->graph);
   g->graph = fresh;
+  g->sig = sig;  // (a failure above leaves the old frame with its own)
   g->kernels = kernel_nodes(fresh);
   return QBC_OK;
 }

@@ -79,3 +79,32 @@ def test_records_replaced(env, floor50k_scene):  # noqa: F811
         _refused_then_equal(torch, ctx, rig, g, views, gbufs)
     finally:
         g.close()
+
+
+def test_failed_update_keeps_the_refusal(env, floor50k_scene):  # noqa: F811
+    """An update that fails leaves the frame captured before, and with it the
+    refusal to replay it in the changed state."""
+    torch, ctx = env
+    import qubatron_gb300 as qb
+    L = qb._lib
+    s = floor50k_scene
+    upload_scene(ctx, s.nodes, s.colors, s.normals)
+    views = _views()
+    _, outs = _outputs(torch, views)
+    ctx.render_views_ex(views, outs, True, two_pass=True, log=True)
+    g = ctx.graph_capture(views, outs, two_pass=True, proposals=L.PROPOSE_LOGGED)
+    try:
+        g.launch()
+        ctx.render_views_ex(views[:1], outs[:1], True, two_pass=True, log=True)  # the log is of other views now
+        ctx.set_option(L.OPT_SERVICE_MIN, 7)
+        with pytest.raises(qb.QbcError):
+            g.update(views)
+        with pytest.raises(qb.QbcError) as e:
+            g.launch()
+        assert e.value.code == -4 and "qbc_graph_launch" in str(e.value)
+        ctx.render_views_ex(views, outs, True, two_pass=True, log=True)
+        g.update(views)
+        g.launch()
+        ctx.synchronize()
+    finally:
+        g.close()
