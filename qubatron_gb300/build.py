@@ -18,7 +18,7 @@ OUT_DIR = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT_DIR, "libqbcuda.so")
 
 SOURCES = ["qbcuda.cu", "frame.cu", "proposal.cu", "build.cu", "boxes.cu", "mlp.cu", "host.cpp"]
-HEADERS = ["trace.cuh", "walker.cuh", "walker_fast.cuh", "share.cuh", "render.cuh", "boxes.cuh", "qbc_internal.h", "qbc_ctx.h", "kernel_index.h", "mlp.h", "mlp_device.cuh", "umma.cuh"]
+HEADERS = ["trace.cuh", "walker.cuh", "walker_fast.cuh", "share.cuh", "render.cuh", "boxes.cuh", "qbc_internal.h", "qbc_ctx.h", "kernel_index.h", "table_state.h", "mlp.h", "mlp_device.cuh", "umma.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_103a,code=sm_103a",

@@ -635,7 +635,7 @@ int build_reserve(BuildScratch* s, int64_t n, int levels) {
     for (int t = 0; t < 3 && !rc; ++t) rc = grow_buf(&s->tab[t], 0, 8 * m, "creator tables");
     if (rc) return rc;
     s->tab_points = m;
-    s->dirty = true;  // emptied on the build's stream
+    s->tables.replaced();  // emptied on the build's stream
   }
   const int64_t nb = scan_chunks_most(n);
   if (s->blocks < nb || !s->blocksum) {
@@ -753,12 +753,14 @@ int build_tree_async(const float* d_pts, const int32_t* d_octets, int64_t n, flo
   const int64_t L0 = *launches;
   int rc = keys_and_prefixes(d_pts, d_octets, n, basesize, levels, s, nullptr, err, stream, grid, launches);
   if (rc) return rc;
-  if (levels > kDense && s->dirty) {
+  const bool tables = levels > kDense, reset = s->tables.begin(tables);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (reset) {
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) return fail(QBC_E_CUDA, "tree build: capture status");
     for (int t = 0; t < 3; ++t)
       if (cudaMemsetAsync(s->tab[t], 0xFF, (size_t)8 * s->tab_points * sizeof(uint32_t), stream) != cudaSuccess)
         return fail(QBC_E_CUDA, "tree build: reset creator tables");
   }
-  s->dirty = true;
   table_levels(n, levels, true, s, stream, grid, launches);
   count_nodes(n, levels, s, false, total, stream, launches);
   write_tree(n, levels, first_index, s, false, true, build_node_bound(n, levels), child, model, rec, stream, launches);
@@ -767,7 +769,7 @@ int build_tree_async(const float* d_pts, const int32_t* d_octets, int64_t n, flo
     *launches = L0;
     return fail(QBC_E_CUDA, "tree build: %s", cudaGetErrorString(e));
   }
-  s->dirty = false;
+  s->tables.end(tables, reset, capture != cudaStreamCaptureStatusNone);
   return QBC_OK;
 }
 

@@ -6,6 +6,7 @@
 #include <cstdint>
 
 #include "qbcuda.h"
+#include "table_state.h"
 
 namespace qbc {
 
@@ -47,7 +48,7 @@ struct BuildScratch {
   int32_t* blocksum = nullptr;
   uint4* box = nullptr;      // boxes of nodes with siblings, 6 x 21 bits
   uint32_t* arrived = nullptr;  // children done, 4 bits a node
-  bool dirty = false;        // tables new, or left by a build that stopped midway: to be emptied
+  TableState tables;         // whether tab's entries are empty
   uint64_t generation = 0;   // raised whenever an array is replaced: captured builds hold their addresses
 };
 
