@@ -678,7 +678,9 @@ struct Shader {
         rq[kRecLogLit] = lit != 0.0f ? 1u : 0u;
         if (wave.pixlog) wave.pixlog[pixel_index()] = lit != 0.0f ? -1.0f : lt;
       }
-      if (shade_bytes(lit)) return false;
+      // (not beside the shader's own walk of an exact basecube, whose kernels
+      // it makes spill: views without boxes 2 % slower, with two trees 4 %)
+      if (!(EXACT && WALK == kWalkExact) && shade_bytes(lit)) return false;
       return flare_or_finish(shade(lit), rp, rd);
     }
     // flare ray ended (octree_fsh.c:456-458)
@@ -735,6 +737,17 @@ constexpr int kStepsPerLook = 6;
 // than lanes share from the start, and sooner is better there: 1000 rays 130
 // us a call with 2 steps, 139 with 4, 143 with 8 (188 without sharing).
 constexpr int kRaySteps = 8, kSpreadSteps = 2;
+
+// The ray of Walker as the compiler must take it in a loop over steps: not
+// known to stay the same. Else the terms of p, d and inv that every step makes
+// from them are held across the loop, and the kernels of an exact basecube
+// spill them (52-116 bytes; the ray queries take 112 and 123 registers).
+// Without leaf boxes, 4 views of 1280x720 of a 2M-point room 8.7 ms with the
+// terms held, 7.2 so; with a second tree 10.7 and 8.5; 2M rays 3.95 and 3.19.
+template <class W>
+__device__ __forceinline__ void reload_ray(W& w) {
+  asm volatile("" : "+f"(w.p.x), "+f"(w.p.y), "+f"(w.p.z), "+f"(w.d.x), "+f"(w.d.y), "+f"(w.d.z));
+}
 
 // MODE kFused: every pixel's primary ray, shadow ray, shading and flare.
 // MODE kPrimaryPass: primary rays only; shaded and flare pixels go to the
@@ -910,6 +923,7 @@ __global__ void __launch_bounds__(kThreads, render_min_blocks<EXACT, DYN, MODE, 
     for (int k = 0; k < kStepsPerLook; ++k) {
       if (S.running) {
         int r;
+        if constexpr (EXACT && WALK == kWalkExact) reload_ray(S.w);
         if constexpr (WALK == kWalkExact) r = S.w.step(sc, S.maxlevel, S.bc, S.st, fast);
         else r = S.w.step(sc, S.maxlevel, S.bc, S.st, [&] { return S.ray_dir(); });
         if (r != kRunning) {
@@ -1084,6 +1098,7 @@ __global__ void __launch_bounds__(kThreads, WALK == kWalkFast ? 6 : 1) rays_kern
 #pragma unroll 1
     for (int k = job.spread ? kSpreadSteps : kRaySteps; k > 0; --k) {
       if (running) {
+        if constexpr (EXACT && WALK == kWalkExact) reload_ray(w);
         if constexpr (WALK == kWalkExact) r = w.step(sc, job.maxlevel, job.bc, st, fast);
         else r = w.step(sc, job.maxlevel, job.bc, st, ray_dir);
         if (r != kRunning) {
