@@ -385,6 +385,8 @@ def time_steps(fn, stream, flush, warmup: int, steps: int):
 
 
 PROPOSAL_WORKLOAD = "floor1m_mlp_1920x1080x16"
+# what a ratio to the plain schedule compares besides the schedules
+SIMPLE_WALK = "in the shader's own arithmetic; the persistent arms walk by t where cubes and leaf boxes allow it"
 
 
 def proposal_comparison(args, device: int, stream, flush) -> dict:
@@ -528,6 +530,7 @@ def proposal_comparison(args, device: int, stream, flush) -> dict:
             "learned_fixed_speedup_vs_plain_two_pass": res["plain_two_pass"]["ms_per_frame"]
             / res["learned_fixed"]["ms_per_frame"],
             "persistent_speedup_vs_plain_simple": res["plain_simple"]["ms_per_frame"] / res["plain_fused"]["ms_per_frame"],
+            "plain_simple_walk": SIMPLE_WALK,
             "network_switched_off_by_autotuner": tuned_gate == 1000,
             "shadow_rays": two["shadow_rays"], "shadow_visits_plain": two["shadow_visits"],
             "cpu_oracle": {k: v for k, v in sample.items() if k not in ("seconds", "rays", "parity")},
@@ -966,7 +969,8 @@ def run_gpu(args):
         proposal["sweep"] = proposal_sweep(ctx, qb, views, outs, stream, update, args)
 
     # the same frames on the plain one-thread-per-pixel schedule (no
-    # persistent queue, no batched ray starts), same tuning otherwise
+    # persistent queue, no batched ray starts), same tuning otherwise; it
+    # keeps the walk in the shader's own arithmetic
     ctx.set_option(qb._lib.OPT_PERSISTENT, 0)
     simple_ms, _, _ = timed(as_graph({}) if use_graph else render_plain)
     ctx.set_option(qb._lib.OPT_PERSISTENT, 1)
@@ -974,7 +978,8 @@ def run_gpu(args):
                     "ms_per_step": statistics.mean(simple_ms),
                     "speedup_of_value": statistics.mean(simple_ms) / statistics.mean(step_ms),
                     "schedule": "one thread per pixel for its whole life, one warp per 32-pixel tile "
-                                "(QBC_OPT_PERSISTENT 0)"}
+                                "(QBC_OPT_PERSISTENT 0)",
+                    "walk": SIMPLE_WALK}
 
     update_ms = None
     if chars:

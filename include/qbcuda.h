@@ -17,6 +17,11 @@
  *    context of the reference.
  *  - Output rows run bottom-up (row 0 is the bottom row), as glReadPixels
  *    returns a GL framebuffer.
+ *  - A context keeps its working memory between calls and gives it back in
+ *    qbc_destroy: on the device the largest host-output frame or ray query
+ *    and the largest dynamic build so far, up to 256 MB for uploads and up to
+ *    256 MB for removals, leaf-box builds and network calls (a call that needs
+ *    more frees it at its end); 512 KB of pinned host memory.
  */
 #ifndef QBCUDA_H
 #define QBCUDA_H
@@ -233,8 +238,9 @@ int qbc_render_views(qbc_ctx* ctx, const qbc_view* views, const qbc_outputs* out
  *   isp     4 floats: entry point of the leaf cell (x, y, z, t)
  *   col,nrm 4 floats each: colour and normal the shader fetches at the leaf
  *   visits  2 uint32: node visits (static, dynamic)
- * pos and dir are n float3; all arrays are host memory when on_device is 0,
- * device memory otherwise.
+ * pos and dir are n float3; all arrays are host memory when on_device is 0
+ * (read and written in stream order; the call waits for its results), device
+ * memory otherwise.
  */
 typedef struct qbc_ray_hits
 {
@@ -511,7 +517,8 @@ int qbc_proposal_set_params(qbc_ctx* ctx, const float* params);
  * row: the 3 proposed t, the occlusion logit). */
 int qbc_proposal_eval(qbc_ctx* ctx, const float* x, int64_t m, float* out);
 /* Mean training loss and its gradient (QBC_PROPOSAL_PARAMS floats) for m host
- * rows: features x (45 each), target t and kind (1 occluded at t, 0 lit). */
+ * rows, at most 8388480: features x (45 each), target t and kind (1 occluded
+ * at t, 0 lit). */
 int qbc_proposal_gradient(qbc_ctx* ctx, const float* x, const float* t, const int8_t* kind, int64_t m, float* loss, float* grad);
 
 /* Run the context's work on this CUDA stream (a cudaStream_t; NULL = the
@@ -522,8 +529,9 @@ int qbc_synchronize(qbc_ctx* ctx);
 /*
  * Tuning options of a context (performance only; results do not change).
  *   QBC_OPT_SERVICE_MIN  1..32, default 4: in the persistent render kernel a
- *   lane whose ray ended waits until this many lanes of its warp wait (or no
- *   ray runs) before the warp starts their next rays together.
+ *   lane whose ray ended waits until the warp, which looks every six steps,
+ *   finds this many of its lanes waiting (or no ray running) and starts their
+ *   next rays together.
  *   QBC_OPT_PROPOSAL_GATE  0..1000 per mille, default 500: QBC_PROPOSE_MLP
  *   tries a pixel's proposals only when the network's occlusion probability
  *   is at least this (0: always; 1000: never, and the network is not run:
@@ -545,9 +553,11 @@ int qbc_synchronize(qbc_ctx* ctx);
  *   persistent kernel (warps take tiles of all views from a work queue and
  *   start new rays in batches), or, with 0, on the plain schedule: one
  *   thread per pixel for the pixel's whole life, one warp per 32-pixel tile,
- *   one launch of tiles_total / 4 blocks. Same pixels; the plain schedule is
- *   the baseline the persistent kernel is measured against. Two-pass renders
- *   always run persistent.
+ *   one launch of tiles_total / 4 blocks. Same pixels. The plain schedule
+ *   keeps the walk in the shader's own arithmetic (which persistent frames
+ *   take where cubes are inexact or leaf boxes not usable), so against a
+ *   persistent frame on the walk by t it differs by schedule and walk.
+ *   Two-pass renders always run persistent.
  *   QBC_OPT_SPLIT_TREES  0 (default) or 1: with 1, a persistent fused frame
  *   with a dynamic tree whose leaf boxes are built (QBC_OPT_BOX_PRUNE 1,
  *   exactly representable cubes) runs as two launches: a one-tree kernel

@@ -24,14 +24,13 @@
 // the boxes unusable.
 //
 // The level counts stay on the device: every kernel finds its level's range
-// from them, and the host reads them once, when all is queued (it read them
-// after every level before). A node's children are neighbours in the order,
-// so their boxes are read in one run, and a level's boxes and records are
-// made in one kernel. 2.6M nodes of a 1M-point floor: 1.1 ms of kernels, 13
-// waits and five allocations before; 0.47 ms of kernels then, 0.41 with the
-// order's positions reserved per block and a node's boxes read together. What
-// is left: the 64-byte records and 32-byte blocks of a level lie scattered
-// (0.3M-0.6M nodes take 20-40 us), and 36 launches, most of small levels.
+// from them, and the host reads them once, when all is queued. A node's
+// children are neighbours in the order, so their boxes are read in one run,
+// and a level's boxes and records are made in one kernel. What bounds it, at
+// 0.41 ms of kernels for 2.6M nodes of a 1M-point floor (1.1 with a host wait
+// per level, boxes and records in passes of their own): the 64-byte records
+// and 32-byte blocks of a level lie scattered (0.3M-0.6M nodes take 20-40 us),
+// and 37 launches, most of small levels.
 
 #include <cuda_runtime.h>
 

@@ -40,13 +40,11 @@
 // galloping search. A static build, which waits for its node count anyway,
 // looks at the order first.
 //
-// 20M points of a room nearly in path order, 52M nodes: 15 ms of kernels
-// before (the boxes in 12 passes over all points with 64-bit divisions, 7.7
-// ms; node writes out of order 2.5; 13 table passes 2.7; 36 divisions a point
-// for its key 0.5) and 3 ms of allocations; 4.8 ms of kernels now (climb 2.2,
-// bound by its chain of loads; tables 1.7; blocks 0.4; keys 0.3) and 0.4 of
-// allocations. The nodes and records alone are 5.2 GB, 0.8 ms. Boxes by one
-// pass a level without atomics: 3.2 ms instead of the climb's 2.6 then.
+// What bounds it: 20M points of a room nearly in path order, 52M nodes, take
+// 4.8 ms of kernels (climb 2.1, its chain of dependent loads; tables 1.7, L2
+// atomics; blocks 0.4; keys 0.3) and 0.4 of allocations, where writing the
+// nodes and records alone, 5.2 GB, takes 0.8. Boxes by a pass over all points
+// per level took 7.7 ms, by one pass a level over nodes 3.2.
 
 #include <cuda_runtime.h>
 
@@ -875,8 +873,8 @@ namespace {
 // the batch equals sequential calls once duplicates of a leaf are resolved:
 // the first in input order removes it, the later ones find the link cut. The
 // points claim their leaves in a hash table of at least twice their number
-// (leaf << 32 | smallest point index), which replaced a sort of all points
-// with its allocations: 20K removals took 0.25 ms, 0.03 now.
+// (leaf << 32 | smallest point index): 0.03 ms for 20K removals, 0.25 by a
+// sort of all points with its allocations.
 constexpr uint64_t kFree = ~0ull;
 
 __device__ __forceinline__ uint64_t claim_slot(int32_t leaf, uint64_t mask) {

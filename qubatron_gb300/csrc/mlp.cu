@@ -560,7 +560,10 @@ int Net::sync_weights(cudaStream_t s) {
 template <class Src>
 int Net::partials(const Src& src, int64_t rows, int* blocks, cudaStream_t s) {
   if (!ready) return fail(QBC_E_STATE, "mlp: not initialised");
-  if (rows > 65535ll * kUmmaRows) return fail(QBC_E_ARG, "mlp gradient: %lld rows exceed one launch", (long long)rows);
+  // (the interface's limit; rows and tiles are 32-bit in the kernel)
+  constexpr int64_t kMostRows = 65535ll * kUmmaRows;
+  if (rows > kMostRows)
+    return fail(QBC_E_ARG, "mlp gradient: %lld rows, at most %lld a call", (long long)rows, (long long)kMostRows);
   if (!partial) {
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);

@@ -85,9 +85,10 @@ __device__ __forceinline__ float4 camera_ray(const qbc_view& v, int i, int j) {
 }
 
 // Whether the pixel is certainly outside the flare cone, without the square
-// root and divisions of the cosine: its approximate cosine c = n.v / |v| is
-// below the threshold by 1e-4, hundreds of times the rounding errors of the
-// exact one (unit n; any other n, or a threshold of 1e-4 or less, says no).
+// root and divisions of the cosine: n.v / |v| is below the threshold by 1e-4,
+// hundreds of times the rounding errors of the exact one. Those scale with
+// |n|, so n need not be a unit vector, only shorter than 1.41 (a longer one,
+// or a threshold of 1e-4 or less, says no).
 __device__ __forceinline__ bool flare_far(const qbc_view& v, float3 csv) {
   const float3 n = make_float3(v.ncamlight[0], v.ncamlight[1], v.ncamlight[2]);
   const float c = v.flare_cos - 1.0e-4f, a = dot3(n, csv), l = dot3(csv, csv);
@@ -711,19 +712,17 @@ __device__ __forceinline__ int tile_view(const Batch& b, int tile) {
   return lo;
 }
 
-// The service phase took a quarter of a frame's instructions at the default
-// threshold (a service every 6 warp steps): basecube entries with six face
-// hits, the cosine of every pixel's flare test, a tile's division by its row
-// length per refill, three normalisations per shaded pixel. The entry now
-// follows from t (FastWalker::start), the flare test first looks at a bound
-// (flare_far), the division runs once per tile and byte outputs are shaded by
-// reciprocal square roots (shade_bytes): 16 x 1080p of a 20M-point room 44.7
-// -> 38.2 ms, a 2M-point character's views 9.2 -> 7.0 ms.
+// The service phase is a quarter of a frame's instructions (it runs for some
+// eight lanes at a time), so it is kept short: the basecube entry follows from
+// t (FastWalker::start) instead of six face hits, the flare test first looks
+// at a bound (flare_far), a tile's division by its row length runs once per
+// tile, and byte outputs are shaded by reciprocal square roots (shade_bytes).
+// Together these took 15 % off 16 x 1080p of a 20M-point room.
 //
-// Lanes whose ray ended wait until at least batch.service_min lanes of the
-// warp need service (or no ray is left running); then ray transitions,
-// refills and ray starts run for all of them together instead of one lane at
-// a time.
+// Lanes whose ray ended wait until a look at the warp, every kStepsPerLook
+// steps, finds at least batch.service_min lanes that need service (or no ray
+// left running); then ray transitions, refills and ray starts run for all of
+// them together instead of one lane at a time.
 constexpr int kServiceMinDefault = 4;
 // Steps a warp takes between two looks at how many of its lanes wait. More
 // steps make fewer and fuller services (and fewer votes), fewer leave fewer
@@ -955,9 +954,11 @@ __global__ void __launch_bounds__(kThreads, render_min_blocks<EXACT, DYN, MODE, 
 // The plain schedule (QBC_OPT_PERSISTENT 0): one thread per pixel for its
 // whole life (primary ray, shadow ray, shading, flare), one warp per 32-pixel
 // tile, no work queue and no batched service; a lane whose pixel is done
-// idles until its warp's last pixel is. Same walker and shader code as
-// render_kernel, so the same pixels; kept as the baseline the persistent
-// kernel is measured against.
+// idles until its warp's last pixel is. Same pixels as render_kernel, with the
+// walk of walker.cuh whatever boxes there are: where render_kernel walks by t,
+// the two differ by schedule and walk. On walker.cuh's walk both, 16 x 1080p
+// of a 1M-point floor take 24.3 ms here and 17.8 there, of a 20M-point room
+// 95.1 and 57.0; render_kernel's walk by t makes these 10.1 and 34.0.
 template <bool EXACT, bool DYN>
 __global__ void __launch_bounds__(kThreads, render_min_blocks<EXACT, DYN, kFused, kWalkExact>()) simple_kernel(DevScene sc, const __grid_constant__ Batch batch) {
   extern __shared__ uint32_t smem[];

@@ -13,20 +13,18 @@
 // shader's arithmetic from the exact entry point, for this cube and the
 // subtree below it (0.05-0.2 % of the visits).
 //
-// What bounds it: the ALU pipe (71 % busy) and instruction issue (68 % of the
-// cycles; DRAM below 2 % of its rate). With the exact subnode test, filter
-// and descent a 1920x1080 view of a 5M-point room took 4.4G warp
-// instructions; this walk takes 3.0G. A step has no divergent branch but the
-// ambiguous one: all four list entries are read and tested at once, the two
-// bounds of an axis in one packed FMA, and a descent reads its own list back
-// from the stack as a pop does (with branches around both, a view took 4.2
-// ms; without, 3.9). 16 x 1080p of a 20M-point room: 68.8 -> 44.7 ms, 37.8
-// with the service phase of render.cuh lightened as well, 32 with that phase
-// looked for every six steps and the list's bit arithmetic shortened (octet
-// bits carried in the t values' low bits); 4M random rays 5.7 -> 4.0 ms. 6
-// blocks of 128 threads per SM (80 registers); 7 (18 bytes spilled) measured
-// the same, 8 spill 94 bytes and take 1.6x. Prefetching the next node's
-// record cost 3 % of a frame and half as much again of random rays.
+// What bounds it: instruction issue (70 % of the cycles) and the ALU pipe (69 %
+// busy; DRAM 2 % of its rate): a 1920x1080 view of a 5M-point room takes 2.69G
+// warp instructions for 201M node visits. A step has no divergent branch but
+// the ambiguous one: all four list entries are read and tested at once, the
+// two bounds of an axis in one packed FMA, the octet bits are carried in the
+// t values' low bits, and a descent reads its own list back from the stack as
+// a pop does (branches around the reads and the descent cost 8 %). Against
+// walker.cuh's walk in the same kernel, 16 x 1080p of a 20M-point room take
+// 34.0 instead of 57.0 ms; 2M random rays in a 2M-point room 1.52 instead of
+// 2.57. 6 blocks of 128 threads per SM (80 registers); 7 (18 bytes spilled)
+// measured the same, 8 spill 94 bytes and take 1.6x. Prefetching the next
+// node's record cost 3 % of a frame and half as much again of random rays.
 //
 // Path. The corner of the current cube is held per axis as the float 1 + path
 // bits (bit 22 - k for level k), so fma(X, S, -S) is the exact coordinate, a
