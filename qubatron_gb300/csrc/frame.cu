@@ -105,6 +105,10 @@ namespace {
 
 int capture_frame(qbc_graph* g, const qbc_view* views, cudaGraph_t* out) {
   qbc_ctx* c = g->ctx;
+  // (a recorded update has built nothing: where the capture fails, the tree
+  // is still the one from before)
+  const DevTreeBuf tree = c->tree[1];
+  const int64_t normals = c->model[1].n_nrm;
   QBC_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
   int rc = g->has_update ? dynamic_update(c, &g->update) : QBC_OK;
   if (!rc) rc = render_views_impl(c, views, g->outs.data(), g->n, 1, g->has_opts ? &g->opts : nullptr, nullptr);
@@ -113,6 +117,11 @@ int capture_frame(qbc_graph* g, const qbc_view* views, cudaGraph_t* out) {
   if (rc || e != cudaSuccess) {
     if (graph) cudaGraphDestroy(graph);
     cudaGetLastError();
+    c->tree[1].n = tree.n;
+    c->tree[1].count_on_device = tree.count_on_device;
+    c->tree[1].box_valid = tree.box_valid;
+    c->tree[1].box_depth = tree.box_depth;
+    c->model[1].n_nrm = normals;
     return rc ? rc : cuda_fail(e, "frame capture");
   }
   *out = graph;

@@ -108,3 +108,36 @@ def test_failed_update_keeps_the_refusal(env, floor50k_scene):  # noqa: F811
         ctx.synchronize()
     finally:
         g.close()
+
+
+def test_failed_update_keeps_the_tree(env, floor50k_scene):  # noqa: F811
+    """... and the dynamic tree uploaded since, which the recorded update would
+    have replaced: its node count and its frames are still those."""
+    torch, ctx = env
+    import qubatron_gb300 as qb
+    L = qb._lib
+    s = floor50k_scene
+    upload_scene(ctx, s.nodes, s.colors, s.normals)
+    p = np.random.default_rng(4).uniform(0.3 * S, 0.7 * S, (40_000, 3)).astype(np.float32)
+    big = qb.build_octree(p, S, LEVELS)
+    ctx.upload_octree(True, big)  # the tree's buffers hold it from now on
+    rig, views = Rig(torch, ctx, n=2000), _views()
+    _, outs = _outputs(torch, views)
+    rig.pose(torch, 0)
+    ctx.dynamic_update(rig.update)
+    ctx.render_views_ex(views, outs, True, two_pass=True, log=True)
+    g = ctx.graph_capture_dynamic(rig.update, views, outs, two_pass=True, proposals=L.PROPOSE_LOGGED)
+    try:
+        ctx.upload_model(True, rig.ch.colors[:1].repeat(40_000, 0), rig.ch.rest_normals[:1].repeat(40_000, 0))
+        ctx.upload_octree(True, big)
+        want = [f.arrays for f in ctx.render_host(views, ("rgba8", "flags", "leaf"))]
+        ctx.render_views_ex(views[:1], outs[:1], True, two_pass=True, log=True)  # the log is of other views now
+        with pytest.raises(qb.QbcError):
+            g.update(views)
+        assert ctx.tree_nodes(1) == big.shape[0] and ctx.model_points(1) == 40_000
+        got = [f.arrays for f in ctx.render_host(views, ("rgba8", "flags", "leaf"))]
+        for a, b in zip(got, want):
+            for k in a:
+                assert np.array_equal(a[k], b[k]), k
+    finally:
+        g.close()
