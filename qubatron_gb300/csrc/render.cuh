@@ -311,7 +311,10 @@ enum Walk : int { kWalkExact = 0, kWalkFast = 1, kWalkFastInstr = 2 };
 template <bool EXACT, bool DYN, bool PROP, int WALK>
 using WalkerOf = std::conditional_t<WALK == kWalkExact, Walker<EXACT, DYN, PROP>, FastWalker<DYN, WALK == kWalkFastInstr, PROP>>;
 
-template <bool EXACT, bool DYN, int MODE, bool PROP, int WALK>
+// BYTES: byte outputs alone may be shaded by shade_bytes(). Not in the
+// persistent kernels of the shader's own walk of an exact basecube, which it
+// makes spill: views without boxes 2 % slower, with two trees 4 %.
+template <bool EXACT, bool DYN, int MODE, bool PROP, int WALK, bool BYTES = !(EXACT && WALK == kWalkExact)>
 struct Shader {
   const DevScene& sc;
   const Batch& batch;
@@ -679,9 +682,7 @@ struct Shader {
         rq[kRecLogLit] = lit != 0.0f ? 1u : 0u;
         if (wave.pixlog) wave.pixlog[pixel_index()] = lit != 0.0f ? -1.0f : lt;
       }
-      // (not beside the shader's own walk of an exact basecube, whose kernels
-      // it makes spill: views without boxes 2 % slower, with two trees 4 %)
-      if (!(EXACT && WALK == kWalkExact) && shade_bytes(lit)) return false;
+      if (BYTES && shade_bytes(lit)) return false;
       return flare_or_finish(shade(lit), rp, rd);
     }
     // flare ray ended (octree_fsh.c:456-458)
@@ -957,8 +958,8 @@ __global__ void __launch_bounds__(kThreads, render_min_blocks<EXACT, DYN, MODE, 
 // idles until its warp's last pixel is. Same pixels as render_kernel, with the
 // walk of walker.cuh whatever boxes there are: where render_kernel walks by t,
 // the two differ by schedule and walk. On walker.cuh's walk both, 16 x 1080p
-// of a 1M-point floor take 24.3 ms here and 17.8 there, of a 20M-point room
-// 95.1 and 57.0; render_kernel's walk by t makes these 10.1 and 34.0.
+// of a 1M-point floor take 24.1 ms here and 17.8 there, of a 20M-point room
+// 93.8 and 57.0; render_kernel's walk by t makes these 10.1 and 34.0.
 template <bool EXACT, bool DYN>
 __global__ void __launch_bounds__(kThreads, render_min_blocks<EXACT, DYN, kFused, kWalkExact>()) simple_kernel(DevScene sc, const __grid_constant__ Batch batch) {
   extern __shared__ uint32_t smem[];
@@ -967,7 +968,7 @@ __global__ void __launch_bounds__(kThreads, render_min_blocks<EXACT, DYN, kFused
   if (tile >= batch.tiles_total) return;
   constexpr int kW = Walker<EXACT, DYN, false>::kWords;
   const Wave wave{};
-  Shader<EXACT, DYN, kFused, false, kWalkExact> S{sc, batch, wave, Stack{smem + tid, kThreads},
+  Shader<EXACT, DYN, kFused, false, kWalkExact, true> S{sc, batch, wave, Stack{smem + tid, kThreads},
                                       PixRef{smem + kW * batch.max_level * kThreads + tid}};
   S.running = false;
   S.enqueue = false;
